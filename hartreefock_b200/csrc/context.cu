@@ -14,6 +14,7 @@
 
 #include "../../include/hfgpu.h"
 #include "eri_dispatch.cuh"
+#include "eri_group_dispatch.cuh"
 #include "eri_split_dispatch.cuh"
 #include "eri_warp_dispatch.cuh"
 
@@ -66,11 +67,12 @@ static const std::vector<double> &boys_table_host() {
     // the per-order rows (the same products the kernels form when they
     // stage a slice into shared memory)
     const double inv_fact[kBoysTaylor] = {1.0, 1.0, 0.5, 1.0 / 6.0, 1.0 / 24.0, 1.0 / 120.0, 1.0 / 720.0};
-    tab.resize((size_t)kBoysFoldedOff + (size_t)(kMaxLtot + 1) * kBoysFoldedSize);
+    tab.resize((size_t)kBoysStagedOff + (size_t)(kMaxLtot + 1) * kBoysFoldedSize);
     for (int L = 0; L <= kMaxLtot; ++L)
       for (int i = 0; i < kBoysGrid; ++i)
         for (int k = 0; k < kBoysRow; ++k)
-          tab[(size_t)kBoysFoldedOff + (size_t)L * kBoysFoldedSize + boys_swizzle(i, k)] =
+          tab[(size_t)kBoysStagedOff + (size_t)L * kBoysFoldedSize + boys_swizzle(i, k)] =
+              tab[(size_t)kBoysFoldedOff + (size_t)L * kBoysFoldedSize + (size_t)i * kBoysRow + k] =
               k < kBoysTaylor ? tab[(size_t)i * kBoysOrders + L + k] * inv_fact[k]
                               : tab[(size_t)kBoysGrid * kBoysOrders + i];
   });
@@ -96,6 +98,12 @@ struct PairClassList {
   // bucket k is [seg_start[m * kBuckets + k], seg_start[m * kBuckets + k + 1])
   std::vector<int> seg_start;
   int *d_pairs = nullptr;
+  // the same pairs with each segment ordered by (first shell, Q descending):
+  // the bras of a grouped task are neighbours here
+  std::vector<int> gpairs;
+  int *d_gpairs = nullptr;
+  double *d_blocks = nullptr;  // primitive pairs by list position (KetField)
+  int *d_block_off = nullptr;
 };
 
 struct QuartetClass {
@@ -103,6 +111,13 @@ struct QuartetClass {
   int bra_pc, ket_pc;
   std::vector<Task> tasks;
   Task *d_tasks = nullptr;
+  // tasks of the grouped kernel (plain J/K builds of the classes in kGroup;
+  // packed as group_task reads them), their ket masks and running cost
+  std::vector<Task> gtasks;
+  Task *d_gtasks = nullptr;
+  uint2 *d_gmasks = nullptr;
+  size_t ngmasks = 0;
+  std::vector<double> gcost_prefix;
   int64_t shell_quartets = 0, function_quartets = 0, prim_quartets = 0;
   double flops = 0;
   // lane occupancy of the thread-per-quartet layout: primitive quartets the
@@ -139,6 +154,7 @@ struct hfg_ctx {
   std::vector<HostShell> shells;
   int npairs = 0;
   std::vector<int> pair_sa, pair_sb, pair_cls, pair_nprim;
+  std::vector<int> pair_pos;  // position of each pair in its class's list (PairClassList::pairs)
   std::vector<double> pair_Q;
   PairClassList pclass[kNumPairClasses];
   std::vector<QuartetClass> qclasses;
@@ -161,6 +177,7 @@ struct hfg_ctx {
   // from hfg_autotune, else prim_target
   int prim_target = 96;
   int class_prim_target[kNumClasses] = {};
+  int group_min_tasks = kGroupMinTasks;  // HFG_GROUP_MIN_TASKS
   // CUDA graph of the plain direct build (hfg_set_graphs): captured on the
   // second build with the same buffers, stream and settings, replayed after
   bool use_graphs = false;
@@ -196,6 +213,7 @@ struct hfg_ctx {
   PrimPairF *d_primf = nullptr;
   int *d_pair_prim_off = nullptr, *d_pair_nprim = nullptr, *d_pair_sa = nullptr, *d_pair_sb = nullptr;
   int *d_pair_ao_a = nullptr, *d_pair_ao_b = nullptr;
+  int *d_pair_pos = nullptr;  // position of each pair in its class's list
   double *d_pair_AB = nullptr, *d_pair_Q = nullptr, *d_boys = nullptr;
   // work buffers
   double *d_J = nullptr, *d_Ka = nullptr, *d_Kb = nullptr, *d_P = nullptr, *d_Pb = nullptr, *d_Pt = nullptr;
@@ -273,16 +291,23 @@ struct hfg_ctx {
     if (stream) cudaStreamSynchronize(stream);
     for (auto &q : qclasses) {
       cudaFree(q.d_tasks);
+      cudaFree(q.d_gtasks);
+      cudaFree(q.d_gmasks);
       if (q.ev_a) cudaEventDestroy(q.ev_a);
       if (q.ev_b) cudaEventDestroy(q.ev_b);
     }
-    for (auto &p : pclass) cudaFree(p.d_pairs);
+    for (auto &p : pclass) {
+      cudaFree(p.d_pairs);
+      cudaFree(p.d_gpairs);
+      cudaFree(p.d_blocks);
+      cudaFree(p.d_block_off);
+    }
     void *bufs[] = {d_prim,       d_pair_prim_off, d_pair_nprim, d_pair_sa,  d_pair_sb,    d_pair_ao_a, d_pair_ao_b,
                     d_pair_AB,    d_pair_Q,        d_boys,       d_J,        d_Ka,         d_Kb,        d_P,
                     d_Pb,         d_Pt,            d_G,          d_Gb,       d_block,      d_scratch[0], d_shell_ao,
                     d_shell_nf,   d_shell_dmax,    d_counters,   d_prev_P[0], d_prev_P[1], d_prev_G[0], d_prev_G[1],
                     d_dP[0],      d_dP[1],         d_primf,      d_pair_mol, d_mol_nbf,    d_mol_off,   d_mol_active,
-                    d_task_active, d_task_counts, d_queue};
+                    d_task_active, d_task_counts, d_queue,    d_pair_pos};
     for (void *b : bufs) cudaFree(b);
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     for (int i = 0; i < kAux; ++i) {
@@ -342,6 +367,70 @@ static inline int64_t pair_functions(const hfg_ctx *c, int p) {
   return c->pair_sa[p] == c->pair_sb[p] ? (int64_t)na * (na + 1) / 2 : (int64_t)na * nb;
 }
 
+// Grouped tasks of one class (eri_group.cuh): every run of bras with one first
+// shell (same molecule and primitive bucket) against every chunk of kets of a
+// bucket that one of them reaches.  `ends`: per bra position and ket bucket the
+// end of the bra's kets, -1 for none.
+static void build_group_tasks(const hfg_ctx *c, QuartetClass &q, const std::vector<int> &ends,
+                              const std::vector<int> &segmax, const std::vector<int64_t> &kprim, int target,
+                              double prim_cost, double quartet_cost) {
+  const PairClassList &BL = c->pclass[q.bra_pc], &KL = c->pclass[q.ket_pc];
+  const auto &bras = BL.gpairs;
+  // bras per task: as many as leave several tasks for every warp of the GPU
+  const int most = (int)std::max<int64_t>(1, std::min<int64_t>(kGroupMaxBras, (int64_t)q.tasks.size() / (c->num_sms * 96)));
+  q.gtasks.clear();
+  q.gcost_prefix.assign(1, 0.0);
+  q.ngmasks = 0;
+  // long contractions first, so that the light tasks fill the end of the launch
+  std::vector<size_t> order;
+  for (int k = kBuckets - 1; k >= 0; --k)
+    for (size_t seg = k; seg + 1 < BL.seg_start.size(); seg += kBuckets) order.push_back(seg);
+  for (size_t seg : order) {
+    const int mol = (int)(seg / kBuckets);
+    for (int g0 = BL.seg_start[seg], g1; g0 < BL.seg_start[seg + 1]; g0 = g1) {
+      int bmax = 0;
+      for (g1 = g0; g1 < BL.seg_start[seg + 1] && c->pair_sa[bras[g1]] == c->pair_sa[bras[g0]]; ++g1)
+        bmax = std::max(bmax, c->pair_nprim[bras[g1]]);
+      for (int k = kBuckets - 1; k >= 0; --k) {
+        const int s0 = KL.seg_start[mol * kBuckets + k];
+        auto end_of = [&](int g) { return ends[(size_t)c->pair_pos[bras[g]] * kBuckets + k]; };
+        int last = -1;
+        for (int g = g0; g < g1; ++g) last = std::max(last, end_of(g));
+        if (last <= s0) continue;
+        const double work = (double)bmax * segmax[mol * kBuckets + k];
+        int G = 1;
+        while (target > 0 && G < 32 && work / G > target) G <<= 1;
+        const int per_task = 32 / G;
+        // a task stays below about kGroupTaskSteps primitive quartets per lane
+        const int run = std::max(1, std::min(most, (int)(kGroupTaskSteps * G / std::max(1.0, work))));
+        for (int st = s0; st < last; st += per_task) {
+          const int e1 = std::min(st + per_task, last);
+          int lg = 0, m2 = 1;
+          while (m2 < e1 - st) m2 <<= 1;
+          while ((32 >> lg) > m2) ++lg;  // 32 / 2^lg lane groups, at least the task's kets
+          for (int b0 = g0; b0 < g1;) {
+            if (end_of(b0) <= st) {
+              ++b0;
+              continue;
+            }
+            int b1 = b0;  // last reaching bra + 1, at most `most` bras from b0
+            double cost = 0;
+            for (int g = b0; g < g1 && g < b0 + run; ++g)
+              if (const int e = std::min(e1, end_of(g)); e > st) {
+                b1 = g + 1;
+                cost += (double)c->pair_nprim[bras[g]] * (double)(kprim[e] - kprim[st]) * prim_cost + (e - st) * quartet_cost;
+              }
+            q.gtasks.push_back(pack_group_task(b0, st, e1 - st, b1 - b0, lg, (unsigned)q.ngmasks));
+            q.ngmasks += b1 - b0;
+            q.gcost_prefix.push_back(q.gcost_prefix.back() + cost);
+            b0 = b1;
+          }
+        }
+      }
+    }
+  }
+}
+
 // Build per-class quartet task lists with Schwarz screening at `threshold`.
 // Every unordered pair of pairs appears once: for different classes all
 // (bra, ket) combinations, for the same class the kets at positions <= the
@@ -380,6 +469,8 @@ static void build_quartet_classes(hfg_ctx *c, double threshold) {
     // classes (split path: one lane per quartet; warp kernel: one warp per
     // quartet) keep 32 kets per task
     const bool grouped = !kSplit[ci] && !kWarp[ci];
+    // per bra and ket bucket: the end of its kets (grouped tasks)
+    std::vector<int> ends(kGroup[ci] ? bras.size() * kBuckets : 0, -1);
     const int target = c->class_prim_target[ci] > 0 ? c->class_prim_target[ci]
                        : c->class_prim_target[ci] < 0 ? 0 : c->prim_target;
     for (size_t b = 0; b < bras.size(); ++b) {
@@ -402,6 +493,7 @@ static void build_quartet_classes(hfg_ctx *c, double threshold) {
         int64_t end = lo;
         if (same) end = std::min<int64_t>(end, (int64_t)b + 1);
         if (end <= s0) continue;
+        if (kGroup[ci]) ends[b * kBuckets + k] = (int)end;
         int per_task = 32;
         if (grouped && target > 0) {
           const double work = (double)bprim * segmax[mol * kBuckets + k];
@@ -437,6 +529,8 @@ static void build_quartet_classes(hfg_ctx *c, double threshold) {
       }
     }
     q.flops = (double)q.prim_quartets * (pf + boys_geom_flops(ltot)) + (double)q.shell_quartets * hf;
+    if (kGroup[ci] && (int64_t)q.tasks.size() >= (int64_t)c->group_min_tasks * c->num_sms)
+      build_group_tasks(c, q, ends, segmax, kprim, target, pf + boys_geom_flops(ltot), hf);
     if (!q.tasks.empty()) c->qclasses.push_back(std::move(q));
   }
   // largest classes first
@@ -444,11 +538,57 @@ static void build_quartet_classes(hfg_ctx *c, double threshold) {
             [](const QuartetClass &a, const QuartetClass &b) { return a.flops > b.flops; });
 }
 
+// Ket masks of one class's grouped tasks, one warp per task and a lane per
+// ket: the quartets of the build (the Schwarz and triangle tests of the task
+// builder) and those with a primitive quartet that is not far.
+__global__ void group_masks_kernel(const EngineView v, const int *__restrict__ bra_list, const int *__restrict__ ket_list,
+                                   const int *__restrict__ pair_pos, const Task *__restrict__ tasks, int ntasks, int same,
+                                   double threshold, double tfar, uint2 *__restrict__ masks) {
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < ntasks; t += warps) {
+    const GroupTask task = group_task(tasks[t]);
+    const int kpos = task.ket_start + lane;
+    const bool in = lane < task.nket;
+    const int kp = in ? ket_list[kpos] : 0;
+    const double qk = v.pair_Q[kp];
+    const int offk = v.pair_prim_off[kp], npk = v.pair_nprim[kp];
+    for (int b = 0; b < task.nbra; ++b) {
+      const int bp = bra_list[task.bra_start + b];
+      const double qb = v.pair_Q[bp];
+      const bool on = in && qb > 0 && qk >= threshold / qb && (!same || kpos <= pair_pos[bp]);
+      bool near = false;
+      if (on) {
+        const int offb = v.pair_prim_off[bp], npb = v.pair_nprim[bp];
+        for (int ik = 0; ik < npk && !near; ++ik) {
+          const PrimPair &pk = v.prim[offk + ik];
+          for (int ib = 0; ib < npb && !near; ++ib) {
+            const PrimPair &pb = v.prim[offb + ib];
+            const double x = pb.Px - pk.Px, y = pb.Py - pk.Py, z = pb.Pz - pk.Pz;
+            near = !(x * x + y * y + z * z >= tfar * (pb.inv_zeta + pk.inv_zeta));
+          }
+        }
+      }
+      const unsigned mx = __ballot_sync(0xffffffffu, on), my = __ballot_sync(0xffffffffu, near);
+      if (lane == 0) masks[task.mask_off + b] = make_uint2(mx, my);
+    }
+  }
+}
+
 static hfg_status upload_classes(hfg_ctx *c) {
   for (auto &q : c->qclasses) {
-    const hfg_status st = upload(&q.d_tasks, q.tasks);
-    if (st != HFG_OK) return st;
+    hfg_status st = upload(&q.d_tasks, q.tasks);
+    if (st != HFG_OK || (st = upload(&q.d_gtasks, q.gtasks)) != HFG_OK) return st;
+    if (q.gtasks.empty()) continue;
+    HFG_CUDA(cudaMalloc((void **)&q.d_gmasks, q.ngmasks * sizeof(uint2)));
+    const ClassEntry &e = kClasses[q.cls];
+    const int grid = std::max(1, std::min(c->num_sms * 8, ((int)q.gtasks.size() + 7) / 8));
+    group_masks_kernel<<<grid, 256, 0, c->stream>>>(c->view(), c->pclass[q.bra_pc].d_gpairs, c->pclass[q.ket_pc].d_pairs,
+                                                    c->d_pair_pos, q.d_gtasks, (int)q.gtasks.size(), q.bra_pc == q.ket_pc,
+                                                    c->opts.schwarz_threshold, far_T(e.la + e.lb + e.lc + e.ld), q.d_gmasks);
+    HFG_CUDA(cudaGetLastError());
   }
+  HFG_CUDA(cudaStreamSynchronize(c->stream));
   return HFG_OK;
 }
 
@@ -460,6 +600,18 @@ static int grid_for(const hfg_ctx *c, int ntasks, int cls) {
   const int def = c->blocks_per_sm > 0 ? c->blocks_per_sm : (c->use_streams && !c->profiling ? 1 : 4);
   const int bps = c->tuned_bps[cls] > 0 ? c->tuned_bps[cls] : def;
   return std::max(1, std::min(blocks, c->num_sms * bps));
+}
+
+// Grouped launch: one warp per task, taken from the device queue, one block of
+// as many warps as the registers hold per SM.  Smaller blocks measured slower
+// also beside other classes: (H2O)32 / 6-31G* build on concurrent streams
+// 22.2 ms, with blocks of 8 warps 25.0 (one per SM) and 23.5 (two), of 4 warps
+// 26.9; (H2O)16 4.88 against 5.40, 5.19 and 5.75.
+static void launch_grouped(const hfg_ctx *c, const EngineView &v, const ClassLaunch &cl, int cls, int mode,
+                           cudaStream_t s) {
+  const ClassEntry &e = kClasses[cls];
+  const int w = group_warps(e.la, e.lb, e.lc, e.ld);
+  kGroup[cls](v, cl, mode, std::max(1, std::min((cl.ntasks + w - 1) / w, c->num_sms)), s);
 }
 
 // Shard `rank` of `count` of tasks with running cost `prefix` (ntasks + 1
@@ -483,18 +635,24 @@ static void shard_range(const double *prefix, int64_t ntasks, int rank, int coun
 // cost (primitive quartets x the class's recursion and Boys flops, plus its
 // horizontal recursions per quartet) is 1/shard_count of the class's, so
 // shards of uneven task mixes take equal work.
-static ClassLaunch base_launch(const hfg_ctx *c, const QuartetClass &q, bool sharded = false) {
+// `grouped`: the launch runs the grouped kernel (plain J/K builds) and takes
+// the class's grouped tasks.
+static ClassLaunch base_launch(const hfg_ctx *c, const QuartetClass &q, bool sharded = false, bool grouped = false) {
   ClassLaunch cl{};
-  cl.bra_list = c->pclass[q.bra_pc].d_pairs;
+  cl.bra_list = grouped ? c->pclass[q.bra_pc].d_gpairs : c->pclass[q.bra_pc].d_pairs;
   cl.ket_list = c->pclass[q.ket_pc].d_pairs;
-  cl.tasks = q.d_tasks;
-  const int total = (int)q.tasks.size();
+  cl.tasks = grouped ? q.d_gtasks : q.d_tasks;
+  cl.masks = grouped ? q.d_gmasks : nullptr;
+  cl.ket_blocks = c->pclass[q.ket_pc].d_blocks;
+  cl.ket_block_off = c->pclass[q.ket_pc].d_block_off;
+  const int total = (int)(grouped ? q.gtasks.size() : q.tasks.size());
+  const std::vector<double> &prefix = grouped ? q.gcost_prefix : q.cost_prefix;
   cl.task_offset = 0;
   cl.task_stride = 1;
   cl.ntasks = total;
-  if (sharded && c->shard_count > 1 && (int)q.cost_prefix.size() == total + 1) {
+  if (sharded && c->shard_count > 1 && (int)prefix.size() == total + 1) {
     int64_t first = 0, count = 0;
-    shard_range(q.cost_prefix.data(), total, c->shard_rank, c->shard_count, &first, &count);
+    shard_range(prefix.data(), total, c->shard_rank, c->shard_count, &first, &count);
     cl.task_offset = (int)first;
     cl.ntasks = (int)count;
   }
@@ -505,10 +663,17 @@ static ClassLaunch base_launch(const hfg_ctx *c, const QuartetClass &q, bool sha
 // the cost share of a launch in its class (shards report their part of the
 // class's quartet and flop counts)
 static double launch_share(const QuartetClass &q, const ClassLaunch &cl) {
-  if (q.tasks.empty()) return 0.0;
-  if ((int)q.cost_prefix.size() != (int)q.tasks.size() + 1 || q.cost_prefix.back() <= 0)
-    return (double)cl.ntasks / (double)q.tasks.size();
-  return (q.cost_prefix[cl.task_offset + cl.ntasks] - q.cost_prefix[cl.task_offset]) / q.cost_prefix.back();
+  const std::vector<Task> &tasks = cl.masks ? q.gtasks : q.tasks;
+  const std::vector<double> &prefix = cl.masks ? q.gcost_prefix : q.cost_prefix;
+  if (tasks.empty()) return 0.0;
+  if (prefix.size() != tasks.size() + 1 || prefix.back() <= 0) return (double)cl.ntasks / (double)tasks.size();
+  return (prefix[cl.task_offset + cl.ntasks] - prefix[cl.task_offset]) / prefix.back();
+}
+
+// plain FP64 J/K builds of the class run the grouped kernel (kGroupMinTasks)
+static bool uses_group(const hfg_ctx *c, const QuartetClass &q) {
+  if (q.gtasks.empty()) return false;
+  return !c->use_streams || c->profiling || (int64_t)q.tasks.size() >= 2 * (int64_t)c->group_min_tasks * c->num_sms;
 }
 
 __global__ void finalize_rhf(const double *J, const double *K, double *G, int n) {
@@ -706,6 +871,11 @@ __global__ void compact_screened_tasks(const EngineView v, const ClassLaunch cl,
 static hfg_status launch_class(hfg_ctx *c, const QuartetClass &q, const ClassLaunch &cl, int mode, bool ref,
                                int prec, cudaStream_t s, int *launches, int slot = 0) {
   const ClassEntry &e = kClasses[q.cls];
+  if (cl.masks) {
+    launch_grouped(c, c->view(), cl, q.cls, mode, s);
+    ++*launches;
+    return HFG_OK;
+  }
   if (class_on_warp(c, q.cls) && mode != kBlock) {
     kWarp[q.cls](c->view(), cl, mode, ref, prec, 0, s);
     ++*launches;
@@ -789,7 +959,9 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
   // those with a quartet above the threshold (late incremental builds keep
   // a small fraction); the class kernels then take them from the queue
   const bool compact = precise && c->use_compaction && nq > 0;
-  if ((c->use_queue || compact) && nq > 0) {
+  bool grouped = false;
+  for (const QuartetClass &q : c->qclasses) grouped = grouped || (!precise && uses_group(c, q));
+  if ((c->use_queue || compact || grouped) && nq > 0) {
     if ((st = ensure_task_scratch(c)) != HFG_OK) return st;
     HFG_CUDA(cudaMemsetAsync(c->d_queue, 0, nq * sizeof(int), s));
     ++launches;
@@ -810,7 +982,7 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
   c->stats = hfg_stats{};
   for (size_t qi = 0; qi < nq; ++qi) {
     QuartetClass &q = c->qclasses[qi];
-    ClassLaunch cl = base_launch(c, q, true);
+    ClassLaunch cl = base_launch(c, q, true, !precise && uses_group(c, q));
     if (c->profiling) HFG_CUDA(cudaEventRecord(q.ev_a, s));
     cl.Da = Da;
     cl.Db = Db;
@@ -824,7 +996,7 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
     if (cl.ntasks > 0) {
       const cudaStream_t cls_stream = cs.pick(uses_split(c, q.cls));
       ClassLaunch cll = cl;
-      if ((c->use_queue || compact) && !uses_split(c, q.cls)) cll.queue = c->d_queue + qi;
+      if ((c->use_queue || compact || cl.masks) && !uses_split(c, q.cls)) cll.queue = c->d_queue + qi;
       if (compact && !uses_split(c, q.cls)) {
         const int cg = std::max(1, std::min(c->num_sms * 8, (cl.ntasks + 7) / 8));
         compact_screened_tasks<<<cg, 256, 0, cls_stream>>>(c->view(), cl, c->d_task_active + c->task_base[qi],
@@ -962,7 +1134,7 @@ static hfg_status ensure_task_scratch(hfg_ctx *c) {
     c->task_base.assign(nq, 0);
     for (size_t i = 0; i < nq; ++i) {
       c->task_base[i] = (int)total;
-      total += c->qclasses[i].tasks.size();
+      total += std::max(c->qclasses[i].tasks.size(), c->qclasses[i].gtasks.size());
     }
     HFG_CUDA(cudaMalloc((void **)&c->d_task_active, std::max<size_t>(1, total) * sizeof(Task)));
     HFG_CUDA(cudaMalloc((void **)&c->d_task_counts, std::max<size_t>(1, nq) * sizeof(int)));
@@ -1045,11 +1217,11 @@ static hfg_status batch_build(hfg_ctx *c, bool uhf, const double *dPa, const dou
     HFG_CUDA(cudaMemsetAsync(c->d_task_counts, 0, nq * sizeof(int), s));
     for (size_t i = 0; i < nq; ++i) {
       const QuartetClass &q = c->qclasses[i];
-      const int nt = (int)q.tasks.size();
+      const ClassLaunch all = base_launch(c, q, false, uses_group(c, q));
+      const int nt = all.ntasks;
       if (nt == 0) continue;
       const int grid = std::max(1, std::min(c->num_sms * 8, (nt + 255) / 256));
-      compact_active_tasks<<<grid, 256, 0, s>>>(q.d_tasks, nt, c->pclass[q.bra_pc].d_pairs, c->d_pair_mol,
-                                                c->d_mol_active, c->d_task_active + c->task_base[i],
+      compact_active_tasks<<<grid, 256, 0, s>>>(all.tasks, nt, all.bra_list, c->d_pair_mol, c->d_mol_active, c->d_task_active + c->task_base[i],
                                                 c->d_task_counts + i);
       ++launches;
     }
@@ -1069,7 +1241,7 @@ static hfg_status batch_build(hfg_ctx *c, bool uhf, const double *dPa, const dou
   c->stats = hfg_stats{};
   for (size_t qi = 0; qi < c->qclasses.size(); ++qi) {
     auto &q = c->qclasses[qi];
-    ClassLaunch cl = base_launch(c, q, true);
+    ClassLaunch cl = base_launch(c, q, true, uses_group(c, q));
     if (compact) {
       cl.tasks = c->d_task_active + c->task_base[qi];
       cl.task_offset = 0;
@@ -1143,10 +1315,11 @@ static hfg_status batch_build_async(hfg_ctx *c, bool uhf, const double *dPa, con
   launches += 2;
   for (size_t i = 0; i < nq; ++i) {
     const QuartetClass &q = c->qclasses[i];
-    const int nt = (int)q.tasks.size();
+    const ClassLaunch all = base_launch(c, q, false, uses_group(c, q));
+    const int nt = all.ntasks;
     if (nt == 0) continue;
     const int grid = std::max(1, std::min(c->num_sms * 8, (nt + 255) / 256));
-    compact_active_tasks<<<grid, 256, 0, s>>>(q.d_tasks, nt, c->pclass[q.bra_pc].d_pairs, c->d_pair_mol, d_active,
+    compact_active_tasks<<<grid, 256, 0, s>>>(all.tasks, nt, all.bra_list, c->d_pair_mol, d_active,
                                               c->d_task_active + c->task_base[i], c->d_task_counts + i);
     ++launches;
   }
@@ -1159,11 +1332,8 @@ static hfg_status batch_build_async(hfg_ctx *c, bool uhf, const double *dPa, con
   for (size_t qi = 0; qi < nq; ++qi) {
     auto &q = c->qclasses[qi];
     if (q.tasks.empty()) continue;
-    ClassLaunch cl = base_launch(c, q, false);
+    ClassLaunch cl = base_launch(c, q, false, uses_group(c, q));  // ntasks: the bound the grid sizes from
     cl.tasks = c->d_task_active + c->task_base[qi];
-    cl.task_offset = 0;
-    cl.task_stride = 1;
-    cl.ntasks = (int)q.tasks.size();  // bound: the grid sizes from it
     cl.ntasks_dev = c->d_task_counts + qi;
     cl.queue = c->d_queue + qi;
     cl.Da = dPa;
@@ -1175,6 +1345,7 @@ static hfg_status batch_build_async(hfg_ctx *c, bool uhf, const double *dPa, con
     const cudaStream_t cls_stream = cs.pick(false);
     const int mode = uhf ? kJkUhf : kJkRhf;
     if (kWarp[q.cls]) kWarp[q.cls](v, cl, mode, ref, 0, 0, cls_stream);
+    else if (cl.masks) launch_grouped(c, v, cl, q.cls, mode, cls_stream);
     else kClasses[q.cls].launch(v, cl, mode, ref, 0, grid_for(c, cl.ntasks, q.cls), cls_stream);
     ++launches;
     c->stats.shell_quartets += q.shell_quartets;
@@ -1300,6 +1471,8 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
   // tuning: HFG_BLOCKS_PER_SM overrides the grid cap (every block stages the
   // class's Boys table once, so fewer, longer-lived blocks stage it less)
   if (const char *e = std::getenv("HFG_BLOCKS_PER_SM")) ctx->blocks_per_sm = std::max(1, std::atoi(e));
+  // tuning: HFG_GROUP_MIN_TASKS sets the tasks per SM from which a class runs the grouped kernel
+  if (const char *e = std::getenv("HFG_GROUP_MIN_TASKS")) ctx->group_min_tasks = std::max(0, std::atoi(e));
   // tuning: HFG_PRIM_TARGET sets the lane-group target (0: one lane per quartet)
   if (const char *e = std::getenv("HFG_PRIM_TARGET")) ctx->prim_target = std::max(0, std::atoi(e));
   // default kernel per large class: the warp-cooperative kernel where one
@@ -1402,7 +1575,7 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
           const double na = std::pow(2 * al / M_PI, 0.75) * std::pow(4 * al, A.L / 2.0);
           const double nb = std::pow(2 * be / M_PI, 0.75) * std::pow(4 * be, B.L / 2.0);
           const double ca = sh->coefficient[A.prim_off + i] * na, cb = sh->coefficient[B.prim_off + j] * nb;
-          PrimPair pp;
+          PrimPair pp{};
           pp.zeta = al + be;
           pp.inv_zeta = 1.0 / pp.zeta;
           const double P[3] = {(al * A.c[0] + be * B.c[0]) * pp.inv_zeta, (al * A.c[1] + be * B.c[1]) * pp.inv_zeta,
@@ -1417,6 +1590,7 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
           pp.bABy = be * AB[1];
           pp.bABz = be * AB[2];
           pp.K = ca * cb * std::exp(-al * be * pp.inv_zeta * ab2) * sqrt2pi54 * pp.inv_zeta;
+          pp.Kf = pp.K * (std::pow(M_PI, 0.25) / std::sqrt(2.0)) / std::sqrt(pp.zeta);
           prim.push_back(pp);
         }
       pn[p] = (int)prim.size() - poff[p];
@@ -1492,6 +1666,7 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
   // ---- class lists: per molecule, primitive-count buckets, each sorted by
   // Q descending
   const int nmols = ctx->nmol;
+  ctx->pair_pos.assign(np, 0);
   for (int pc = 0; pc < kNumPairClasses; ++pc) {
     PairClassList &L = ctx->pclass[pc];
     L.pairs.clear();
@@ -1508,8 +1683,42 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
       L.pairs.insert(L.pairs.end(), seg[x].begin(), seg[x].end());
     }
     L.seg_start[seg.size()] = (int)L.pairs.size();
-    if ((st = upload(&L.d_pairs, L.pairs)) != HFG_OK) return st;
+    for (size_t x = 0; x < L.pairs.size(); ++x) ctx->pair_pos[L.pairs[x]] = (int)x;
+    L.gpairs = L.pairs;
+    for (size_t x = 0; x < seg.size(); ++x)
+      std::stable_sort(L.gpairs.begin() + L.seg_start[x], L.gpairs.begin() + L.seg_start[x + 1],
+                       [&](int a, int b) { return ctx->pair_sa[a] < ctx->pair_sa[b]; });
+    std::vector<int> segmax_of(L.pairs.size(), 0);
+    for (size_t x = 0; x < seg.size(); ++x) {
+      int most = 0;
+      for (int p : seg[x]) most = std::max(most, pn[p]);
+      std::fill(segmax_of.begin() + L.seg_start[x], segmax_of.begin() + L.seg_start[x + 1], most);
+    }
+    std::vector<int> boff;
+    std::vector<double> blocks;
+    for (size_t x = 0; x < L.pairs.size(); x += 32) {
+      const size_t rec = blocks.size() / kKetStride, end = std::min(x + 32, L.pairs.size());
+      boff.push_back((int)rec);
+      // as many records as the longest contraction of a segment the block
+      // touches: a task's kets are of one segment and read alike
+      int most = 1;
+      for (size_t y = x; y < end; ++y) most = std::max(most, segmax_of[y]);
+      blocks.resize((rec + most) * kKetStride, 0.0);
+      // records past a pair's last one: no weight, at a distance from everything
+      for (size_t r = rec; r < rec + most; ++r)
+        for (int k = 0; k < 32; ++k) blocks[r * kKetStride + kKetPx * 32 + k] = 1e6;
+      for (size_t y = x; y < end; ++y)
+        for (int i = 0; i < pn[L.pairs[y]]; ++i) {
+          const PrimPair &pp = prim[poff[L.pairs[y]] + i];
+          const double f[kKetFields] = {pp.Px, pp.Py, pp.Pz, pp.Kf, pp.inv_zeta, pp.bABx, pp.bABy, pp.bABz, pp.zeta, pp.K};
+          for (int k = 0; k < kKetFields; ++k) blocks[(rec + i) * kKetStride + k * 32 + (y - x)] = f[k];
+        }
+    }
+    if ((st = upload(&L.d_pairs, L.pairs)) != HFG_OK || (st = upload(&L.d_gpairs, L.gpairs)) != HFG_OK ||
+        (st = upload(&L.d_blocks, blocks)) != HFG_OK || (st = upload(&L.d_block_off, boff)) != HFG_OK)
+      return st;
   }
+  if ((st = upload(&ctx->d_pair_pos, ctx->pair_pos)) != HFG_OK) return st;
   build_quartet_classes(ctx.get(), ctx->opts.schwarz_threshold);
   if ((st = upload_classes(ctx.get())) != HFG_OK) return st;
   if (ctx->batch) {
@@ -1918,20 +2127,20 @@ hfg_status hfg_autotune(hfg_ctx *c, const double *dP, int32_t *chosen, int32_t c
   }
   for (auto &q : c->qclasses) {
     if (kSplit[q.cls] || kWarp[q.cls] || q.tasks.empty()) continue;
-    ClassLaunch cl = base_launch(c, q, true);
+    ClassLaunch cl = base_launch(c, q, true, !c->precision_form() && uses_group(c, q));
     if (cl.ntasks == 0) continue;
     cl.Da = dP;
     cl.Dt = dP;
     cl.J = c->d_J;
     cl.Ka = c->d_Ka;
     float best = 1e30f;
-    int best_bps = 4;
+    int best_bps = 4, launches = 0;
     for (int b : cand) {
       c->tuned_bps[q.cls] = b;
-      const int grid = grid_for(c, cl.ntasks, q.cls);
-      kClasses[q.cls].launch(c->view(), cl, kJkRhf, ref, 0, grid, s);
+      if ((st = launch_class(c, q, cl, kJkRhf, ref, 0, s, &launches)) != HFG_OK) return st;
       HFG_CUDA(cudaEventRecord(c->ev0, s));
-      for (int r = 0; r < 2; ++r) kClasses[q.cls].launch(c->view(), cl, kJkRhf, ref, 0, grid, s);
+      for (int r = 0; r < 2; ++r)
+        if ((st = launch_class(c, q, cl, kJkRhf, ref, 0, s, &launches)) != HFG_OK) return st;
       HFG_CUDA(cudaEventRecord(c->ev1, s));
       HFG_CUDA(cudaEventSynchronize(c->ev1));
       HFG_CUDA(cudaGetLastError());
@@ -1965,6 +2174,8 @@ static hfg_status rebuild_tasks(hfg_ctx *c) {
   HFG_CUDA(cudaDeviceSynchronize());  // queued builds may still read the old lists
   for (auto &q : c->qclasses) {
     cudaFree(q.d_tasks);
+    cudaFree(q.d_gtasks);
+    cudaFree(q.d_gmasks);
     if (q.ev_a) cudaEventDestroy(q.ev_a);
     if (q.ev_b) cudaEventDestroy(q.ev_b);
   }
@@ -2021,16 +2232,17 @@ hfg_status hfg_autotune_tasks(hfg_ctx *c, const double *dP, int32_t *chosen, int
     if ((st = rebuild_tasks(c)) != HFG_OK) return st;
     for (auto &q : c->qclasses) {
       if (kWarp[q.cls] || kSplit[q.cls]) continue;  // one warp per quartet: no lane groups
-      ClassLaunch cl = base_launch(c, q, true);
+      ClassLaunch cl = base_launch(c, q, true, !c->precision_form() && uses_group(c, q));
       if (cl.ntasks == 0) continue;
       cl.Da = dP;
       cl.Dt = dP;
       cl.J = c->d_J;
       cl.Ka = c->d_Ka;
-      const int grid = grid_for(c, cl.ntasks, q.cls);
-      kClasses[q.cls].launch(c->view(), cl, kJkRhf, ref, 0, grid, s);
+      int launches = 0;
+      if ((st = launch_class(c, q, cl, kJkRhf, ref, 0, s, &launches)) != HFG_OK) return st;
       HFG_CUDA(cudaEventRecord(c->ev0, s));
-      for (int r = 0; r < 2; ++r) kClasses[q.cls].launch(c->view(), cl, kJkRhf, ref, 0, grid, s);
+      for (int r = 0; r < 2; ++r)
+        if ((st = launch_class(c, q, cl, kJkRhf, ref, 0, s, &launches)) != HFG_OK) return st;
       HFG_CUDA(cudaEventRecord(c->ev1, s));
       HFG_CUDA(cudaEventSynchronize(c->ev1));
       HFG_CUDA(cudaGetLastError());
@@ -2233,13 +2445,14 @@ extern "C" hfg_status hfg_fock_rhf_noalloc(hfg_ctx *c, const double *dP, double 
   const EngineView v = c->view();
   const bool ref = c->opts.eri_convention == HFG_ERI_REFERENCE;
   for (const auto &q : c->qclasses) {
-    ClassLaunch cl = base_launch(c, q);
+    ClassLaunch cl = base_launch(c, q, false, uses_group(c, q));
     cl.Da = dP;
     cl.Dt = dP;
     cl.J = J;
     cl.Ka = K;
     // the large classes run warp-cooperatively: shared memory only, no scratch
     if (kWarp[q.cls]) kWarp[q.cls](v, cl, kJkRhf, ref, 0, 0, s);
+    else if (cl.masks) launch_grouped(c, v, cl, q.cls, kJkRhf, s);
     else kClasses[q.cls].launch(v, cl, kJkRhf, ref, 0, grid_for(c, cl.ntasks, q.cls), s);
   }
   const int fg = std::max(1, std::min(1024, (int)((nn + 255) / 256)));

@@ -17,21 +17,12 @@ namespace hfg {
 template <int N>
 constexpr int kUnrollBlock = N <= 81 ? 64 : 1;
 
-__device__ __forceinline__ double inv_factorial(int k) {
-  // 1/k! for k = 0..6 as a select chain (an indexed array would live in
-  // local memory and be rebuilt on every call)
-  return k <= 1 ? 1.0 : k == 2 ? 0.5 : k == 3 ? 1.0 / 6.0 : k == 4 ? 1.0 / 24.0 : k == 5 ? 1.0 / 120.0 : 1.0 / 720.0;
-}
-
+// Copies the class's prepared Boys slice into shared memory.
 template <int LTOT>
 __device__ __forceinline__ void stage_boys(double *tab, const double *__restrict__ g) {
-  for (int x = threadIdx.x; x < kBoysGrid * kBoysRow; x += blockDim.x) {
-    const int i = x / kBoysRow, k = x - i * kBoysRow;
-    // Taylor coefficients F_{LTOT+k}(T_i)/k!, then e^-T_i from the table's
-    // tail, each at its swizzled place in the row
-    tab[boys_swizzle(i, k)] =
-        k < kBoysTaylor ? g[i * kBoysOrders + LTOT + k] * inv_factorial(k) : g[kBoysGrid * kBoysOrders + i];
-  }
+  const double2 *src = reinterpret_cast<const double2 *>(g + kBoysStagedOff + LTOT * kBoysFoldedSize);
+  double2 *dst = reinterpret_cast<double2 *>(tab);
+  for (int x = threadIdx.x; x < kBoysFoldedSize / 2; x += blockDim.x) dst[x] = __ldg(src + x);
   __syncthreads();
 }
 
@@ -76,8 +67,8 @@ __device__ __noinline__ void boys_edges_fp64(double *F, double T, double scale) 
 // at the switch.  (The far, small quartets that run in FP32 are mostly at
 // large T: the asymptotic branch is their common case.)
 constexpr float kBoysF32Band = 4.0f;
-template <int M>
-__device__ __forceinline__ void boys_eval_f32(float *F, float T, float scale, const double *__restrict__ tab) {
+template <int M, class Tab>
+__device__ __forceinline__ void boys_eval_f32(float *F, float T, float scale, const Tab tab) {
   if (T >= (float)kBoysTmax + kBoysF32Band) {
     const float r = rsqrtf(T);
     float f = 0.88622692545275801365f * r;  // sqrt(pi)/2 / sqrt(T)
@@ -93,11 +84,11 @@ __device__ __forceinline__ void boys_eval_f32(float *F, float T, float scale, co
   } else if (T >= (float)kBoysStep && T < (float)kBoysTmax) {
     const int i = __float2int_rn(T * (float)(1.0 / kBoysStep));
     const float dt = (float)i * (float)kBoysStep - T;
-    const double *t = tab + i * kBoysRow;
-    const int sw = (i >> 1) & 7;
-    float f = (float)t[6 ^ sw];
+    double t[kBoysRow];
+    tab.row(i, t);
+    float f = (float)t[6];
 #pragma unroll
-    for (int k = 5; k >= 0; --k) f = fmaf(f, dt, (float)t[k ^ sw]);
+    for (int k = 5; k >= 0; --k) f = fmaf(f, dt, (float)t[k]);
     float fm[M + 1];
     fm[M] = f;
     if (M > 0) {
@@ -108,7 +99,7 @@ __device__ __forceinline__ void boys_eval_f32(float *F, float T, float scale, co
       x = fmaf(x, dt, 0.5f);
       x = fmaf(x, dt, 1.0f);
       x = fmaf(x, dt, 1.0f);
-      const float e = (float)t[7 ^ sw] * x, t2 = 2.0f * T;
+      const float e = (float)t[7] * x, t2 = 2.0f * T;
 #pragma unroll
       for (int m = M - 1; m >= 0; --m) fm[m] = fmaf(t2, fm[m + 1], e) * (1.0f / (2 * m + 1));
     }
@@ -131,8 +122,8 @@ __device__ __forceinline__ void boys_eval_f32(float *F, float T, float scale, co
 // (ket primitive, bra primitive) grid and the group sums its accumulators
 // with shuffles afterwards (warp-shuffle contraction), so every lane of the
 // group ends with the whole contracted block.  lg is warp-uniform.
-template <int LA, int LB, int LC, int LD, bool REF, class R>
-__device__ __forceinline__ void accumulate_primitives_grouped(const EngineView &v, const double *tab, int bp, int kp,
+template <int LA, int LB, int LC, int LD, bool REF, class R, class Tab>
+__device__ __forceinline__ void accumulate_primitives_grouped(const EngineView &v, const Tab tab, int bp, int kp,
                                                               int npk, R *acc, int lg) {
   constexpr int LTOT = LA + LB + LC + LD;
   using Cls = EriClass<LA, LB, LC, LD, REF>;
@@ -161,7 +152,7 @@ __device__ __forceinline__ void accumulate_primitives_grouped(const EngineView &
       const double PQx = pb.Px - pk.Px, PQy = pb.Py - pk.Py, PQz = pb.Pz - pk.Pz;
       const double T = rho * (PQx * PQx + PQy * PQy + PQz * PQz);
       double F[LTOT + 1];
-      boys_eval<LTOT, double>(F, T, pb.K * pk.K * rs, tab);
+      boys_eval<LTOT>(F, T, pb.K * pk.K * rs, tab);
       const double roz = rho * pb.inv_zeta, ie = pk.inv_zeta;
       Cls::template prim<double>(acc, F, pb.PAx, pb.PAy, pb.PAz, -roz * PQx, -roz * PQy, -roz * PQz,
                                  0.5 * pb.inv_zeta, roz, -(pb.bABx + pk.bABx) * ie, -(pb.bABy + pk.bABy) * ie,
@@ -180,8 +171,8 @@ __device__ __forceinline__ void accumulate_primitives_grouped(const EngineView &
 
 // `acc`: the block's accumulators, a register array (R*) or any indexable
 // accumulator type (lane groups need the register array).
-template <int LA, int LB, int LC, int LD, bool REF, class R, class A>
-__device__ __forceinline__ void accumulate_primitives(const EngineView &v, const double *tab, int bp, int kp, int npk,
+template <int LA, int LB, int LC, int LD, bool REF, class R, class Tab, class A>
+__device__ __forceinline__ void accumulate_primitives(const EngineView &v, const Tab tab, int bp, int kp, int npk,
                                                       A acc, int lg = 0) {
   if constexpr (std::is_pointer<A>::value) {
     if (lg > 0) {
@@ -228,7 +219,7 @@ __device__ __forceinline__ void accumulate_primitives(const EngineView &v, const
         const double PQx = pb.Px - pk.Px, PQy = pb.Py - pk.Py, PQz = pb.Pz - pk.Pz;
         const double T = rho * (PQx * PQx + PQy * PQy + PQz * PQz);
         double F[LTOT + 1];
-        boys_eval<LTOT, double>(F, T, pb.K * pk.K * rs, tab);
+        boys_eval<LTOT>(F, T, pb.K * pk.K * rs, tab);
         const double roz = rho * pb.inv_zeta;
         const double ie = pk.inv_zeta;
         Cls::template prim<double>(acc, F, pb.PAx, pb.PAy, pb.PAz, -roz * PQx, -roz * PQy, -roz * PQz,
@@ -243,8 +234,8 @@ __device__ __forceinline__ void accumulate_primitives(const EngineView &v, const
 // `kp`, components in canonical order, normalisation applied.  `npk` = 0
 // yields an all-zero block (inactive lanes).  R is the arithmetic type
 // (see accumulate_primitives).
-template <int LA, int LB, int LC, int LD, bool REF, class R = double>
-__device__ __forceinline__ void quartet_block(const EngineView &v, const double *tab, int bp, int kp, int npk, R *out,
+template <int LA, int LB, int LC, int LD, bool REF, class R = double, class Tab>
+__device__ __forceinline__ void quartet_block(const EngineView &v, const Tab tab, int bp, int kp, int npk, R *out,
                                               int lg = 0) {
   constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
   using Cls = EriClass<LA, LB, LC, LD, REF>;
@@ -311,8 +302,8 @@ __device__ __forceinline__ bool screen_task(const EngineView &v, const ClassLaun
 // row range the orientation changes the value.  This reproduces the choice
 // per element (AO index == function ID).  Kept out of line: it holds three
 // (dd|dd) blocks and is only reached by the rare two-d-shell quartets.
-template <class R>
-static __device__ __noinline__ void dddd_reference_values(const EngineView &v, const double *tab, int bp, int kp,
+template <class R, class Tab>
+static __device__ __noinline__ void dddd_reference_values(const EngineView &v, const Tab tab, int bp, int kp,
                                                           int npk, R *out) {
   constexpr int N = 6;
   const int sab = v.pair_sa[bp], skt = v.pair_sa[kp];
@@ -345,8 +336,8 @@ static __device__ __noinline__ void dddd_reference_values(const EngineView &v, c
         }
 }
 
-template <int LA, int LB, int LC, int LD, bool REF, class R>
-__device__ __forceinline__ void quartet_values(const EngineView &v, const double *tab, int bp, int kp, int npk,
+template <int LA, int LB, int LC, int LD, bool REF, class R, class Tab>
+__device__ __forceinline__ void quartet_values(const EngineView &v, const Tab tab, int bp, int kp, int npk,
                                                R *out, int lg) {
   if constexpr (REF && LA == 2 && LB == 2 && LC == 2 && LD == 2) {
     dddd_reference_values<R>(v, tab, bp, kp, npk, out);  // single-quartet queries only: lg == 0
@@ -366,13 +357,11 @@ __global__ void __launch_bounds__(32 * fused_warps(LA, LB, LC, LD), fused_min_bl
   constexpr int N = NA * NB * NC * ND;
   static_assert(SCR == kScreenNone || MODE == kJkRhf || MODE == kJkUhf, "screening applies to J/K builds");
   // the class's Boys slice: per-order rows in global memory, or staged
-  __shared__ double tab_sh[boys_from_global(LA, LB, LC, LD) ? 1 : kBoysGrid * kBoysRow];
-  const double *__restrict__ tab = tab_sh;
-  if constexpr (boys_from_global(LA, LB, LC, LD)) {
-    tab = v.boys_table + kBoysFoldedOff + LTOT * kBoysFoldedSize;
-  } else {
-    stage_boys<LTOT>(tab_sh, v.boys_table);
-  }
+  __shared__ __align__(16) double tab_sh[boys_from_global(LA, LB, LC, LD) ? 1 : kBoysGrid * kBoysRow];
+  constexpr bool kGlobal = boys_from_global(LA, LB, LC, LD);
+  if constexpr (!kGlobal) stage_boys<LTOT>(tab_sh, v.boys_table);
+  const std::conditional_t<kGlobal, BoysGlobal, BoysShared> tab{
+      kGlobal ? v.boys_table + kBoysFoldedOff + LTOT * kBoysFoldedSize : tab_sh};
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -572,12 +561,12 @@ template <int LA, int LB>
 __global__ void __launch_bounds__(kThreads) schwarz_kernel(const EngineView v, const int *pairs, int npairs,
                                                            double *Q) {
   constexpr int NA = ncart(LA), NB = ncart(LB);
-  __shared__ double tab[kBoysGrid * kBoysRow];
+  __shared__ __align__(16) double tab[kBoysGrid * kBoysRow];
   stage_boys<2 * (LA + LB)>(tab, v.boys_table);
   for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < npairs; x += gridDim.x * blockDim.x) {
     const int p = pairs[x];
     double out[NA * NB * NA * NB];
-    quartet_block<LA, LB, LA, LB, false>(v, tab, p, p, v.pair_nprim[p], out);
+    quartet_block<LA, LB, LA, LB, false>(v, BoysShared{tab}, p, p, v.pair_nprim[p], out);
     double m = 0.0;
 #pragma unroll
     for (int a = 0; a < NA; ++a)

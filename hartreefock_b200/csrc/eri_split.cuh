@@ -26,8 +26,8 @@ namespace hfg {
 // spills of the large blocks but made the classes 1.3-2x slower: global
 // read-modify-writes per primitive quartet cost more than local-memory
 // spills, which stay in L1)
-template <int LA, int LB, int LC, int LD, bool REF, class R>
-__device__ __forceinline__ void prim_block_to_scratch(const EngineView &v, const double *tab, int bp, int kp, int npk,
+template <int LA, int LB, int LC, int LD, bool REF, class R, class Tab>
+__device__ __forceinline__ void prim_block_to_scratch(const EngineView &v, const Tab tab, int bp, int kp, int npk,
                                                       double *scr, long long stride) {
   using Cls = EriClass<LA, LB, LC, LD, REF>;
   R acc[Cls::kAcc];
@@ -39,8 +39,8 @@ __device__ __forceinline__ void prim_block_to_scratch(const EngineView &v, const
 }
 
 // One quartet's contracted [e0|f0] block(s) in precision R, to its slot.
-template <int LA, int LB, int LC, int LD, bool REF, class R>
-__device__ __forceinline__ void prim_to_scratch(const EngineView &v, const double *tab, int bp, int kp,
+template <int LA, int LB, int LC, int LD, bool REF, class R, class Tab>
+__device__ __forceinline__ void prim_to_scratch(const EngineView &v, const Tab tab, int bp, int kp,
                                                 const SplitChunk &ch, long long slot) {
   constexpr bool kOrient = REF && LA == 2 && LB == 2 && LC == 2 && LD == 2;
   if constexpr (kOrient) {
@@ -62,13 +62,11 @@ template <int LA, int LB, int LC, int LD, bool REF, int SCR = kScreenNone>
 __global__ void __launch_bounds__(kThreads) eri_prim_split_kernel(const EngineView v, const ClassLaunch cl,
                                                                   const SplitChunk ch) {
   constexpr int LTOT = LA + LB + LC + LD;
-  __shared__ double tab_sh[boys_from_global_split(LA, LB, LC, LD) ? 1 : kBoysGrid * kBoysRow];
-  const double *__restrict__ tab = tab_sh;
-  if constexpr (boys_from_global_split(LA, LB, LC, LD)) {
-    tab = v.boys_table + kBoysFoldedOff + LTOT * kBoysFoldedSize;
-  } else {
-    stage_boys<LTOT>(tab_sh, v.boys_table);
-  }
+  __shared__ __align__(16) double tab_sh[boys_from_global_split(LA, LB, LC, LD) ? 1 : kBoysGrid * kBoysRow];
+  constexpr bool kGlobal = boys_from_global_split(LA, LB, LC, LD);
+  if constexpr (!kGlobal) stage_boys<LTOT>(tab_sh, v.boys_table);
+  const std::conditional_t<kGlobal, BoysGlobal, BoysShared> tab{
+      kGlobal ? v.boys_table + kBoysFoldedOff + LTOT * kBoysFoldedSize : tab_sh};
   const long long slot = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (slot >= (long long)ch.ntasks * 32) return;  // whole warps
   const Task task = launch_task(cl, ch.task0 + (int)(slot >> 5));

@@ -335,7 +335,8 @@ def emit_launchers(out_dir):
                       f"    launch_class_{tag}_scr(v, cl, mode, ref, prec, grid, s);",
                       "    return;", "  }"]
         lines.append("  switch (mode) {")
-        for mode in modes:
+        # the large classes' builds run the split or warp kernels
+        for mode in ("kBlock",) if split else modes:
             lines.append(f"    case {mode}:")
             launch(lines, "      ", f"launch_fused<{a}, {b}, {c}, {d}, {mode}, {{r}}>", ref)
             lines.append("      break;")
@@ -922,6 +923,45 @@ def emit_warp(out_dir):
         fh.write("\n".join(lines))
 
 
+def is_group_class(la, lb, lc, ld):
+    """Classes the grouped J/K kernel (eri_group.cuh) serves: contracted blocks
+    of at most 27 elements.  Above that the accumulators it keeps over a run of
+    bras spill: (dp|ps) 0.98 -> 1.17 ms, (dd|ss) 0.31 -> 0.50 per (H2O)32 build,
+    (ds|ds) 0.17 -> 0.22 per (H2O)16 build."""
+    ne = sum((L + 1) * (L + 2) // 2 for L in range(la, la + lb + 1))
+    nf = sum((L + 1) * (L + 2) // 2 for L in range(lc, lc + ld + 1))
+    return ne * nf <= 27
+
+
+def emit_group(out_dir):
+    """One launcher TU per grouped class and the dispatch table kGroup[]."""
+    _, quartets = canonical_classes()
+    tags = [q for q in quartets if is_group_class(*q)]
+    for (a, b, c, d) in tags:
+        lines = [f"// Generated by gen_eri.py: grouped J/K kernels of the ({a}{b}|{c}{d}) class.",
+                 '#include "eri_group.cuh"', '#include "eri_group_dispatch.cuh"', "", "namespace hfg {", "",
+                 f"void launch_group_{a}{b}{c}{d}(const EngineView &v, const ClassLaunch &cl, int mode, int grid, "
+                 "cudaStream_t s) {",
+                 f"  if (mode == kJkUhf) launch_group<{a}, {b}, {c}, {d}, kJkUhf>(v, cl, grid, s);",
+                 f"  else launch_group<{a}, {b}, {c}, {d}, kJkRhf>(v, cl, grid, s);",
+                 "}", "", "}  // namespace hfg", ""]
+        with open(os.path.join(out_dir, f"eri_group_{a}{b}{c}{d}.cu"), "w") as fh:
+            fh.write("\n".join(lines))
+    lines = ["// Generated by gen_eri.py: grouped launcher table.", "#pragma once", '#include "hfg_internal.cuh"', "",
+             "namespace hfg {", "",
+             "using GroupLauncher = void (*)(const EngineView &, const ClassLaunch &, int, int, cudaStream_t);"]
+    for (a, b, c, d) in tags:
+        lines.append(f"void launch_group_{a}{b}{c}{d}(const EngineView &v, const ClassLaunch &cl, int mode, int grid, "
+                     "cudaStream_t s);")
+    lines += ["", "// grouped launcher per class (same order as kClasses), nullptr for the others",
+              "static const GroupLauncher kGroup[] = {"]
+    for q in quartets:
+        lines.append("    %s," % ("launch_group_%d%d%d%d" % q if q in tags else "nullptr"))
+    lines += ["};", "", "}  // namespace hfg", ""]
+    with open(os.path.join(out_dir, "eri_group_dispatch.cuh"), "w") as fh:
+        fh.write("\n".join(lines))
+
+
 if __name__ == "__main__":
     here = os.path.dirname(os.path.abspath(__file__))
     out_dir = sys.argv[1] if len(sys.argv) > 1 else here
@@ -929,3 +969,4 @@ if __name__ == "__main__":
     emit_launchers(out_dir)
     emit_split(out_dir)
     emit_warp(out_dir)
+    emit_group(out_dir)

@@ -13,17 +13,20 @@ constexpr double kBoysStep = 0.05;            // grid spacing in T
 constexpr double kBoysTmax = 36.0;            // above: asymptotic F_0 + upward recursion
 constexpr int kBoysGrid = 721;                // 36 / 0.05 + 1 grid points
 constexpr int kBoysOrders = kMaxLtot + kBoysTaylor;  // orders 0 .. 14 tabulated
-// staged row: 7 Taylor terms and exp(-T_i), 8 doubles.  Word k of row i is
-// stored at k ^ ((i >> 1) & 7) within the row: rows start on bank 0 or 16
-// only, and the swizzle spreads one column of 16 consecutive rows over all
-// 32 banks (plain rows put a whole warp's column on one bank pair).
+// staged row: 7 Taylor terms and exp(-T_i), 8 doubles, read as four 16-byte
+// words.  Word j of row i is stored at j ^ ((i >> 1) & 3) within the row: rows
+// start on one of two halves of the banks only, and the swizzle spreads one
+// word of 8 consecutive rows (the lanes of one 16-byte access phase) over all
+// banks.
 constexpr int kBoysRow = kBoysTaylor + 1;
-__host__ __device__ constexpr int boys_swizzle(int i, int k) { return i * kBoysRow + (k ^ ((i >> 1) & 7)); }
+__host__ __device__ constexpr int boys_swizzle(int i, int k) { return i * kBoysRow + (k ^ (i & 6)); }
 // Per-order rows ready for evaluation, after the e^-T tail of the table:
 // table L (L = 0 .. kMaxLtot) holds in each grid row F_{L+k}(T_i) / k!
-// (k < kBoysTaylor) and e^-T_i, swizzled as boys_swizzle places them.
+// (k < kBoysTaylor) and e^-T_i, unswizzled.
 constexpr int kBoysFoldedOff = kBoysGrid * kBoysOrders + kBoysGrid;
 constexpr int kBoysFoldedSize = kBoysGrid * kBoysRow;
+// the same rows as a staged slice holds them (swizzled), for block-wide copies
+constexpr int kBoysStagedOff = kBoysFoldedOff + (kMaxLtot + 1) * kBoysFoldedSize;
 
 constexpr int kWarpsPerBlock = 4;
 constexpr int kThreads = 32 * kWarpsPerBlock;
@@ -83,6 +86,22 @@ __host__ __device__ constexpr bool boys_from_global_split(int la, int lb, int lc
   return !(la == 2 && lb == 2 && lc == 2 && (ld == 1 || ld == 2));
 }
 
+// T from which a primitive quartet of total angular momentum L counts as far:
+// there the asymptotic F_m = (2m-1)!!/(2T)^m sqrt(pi/T)/2 without the e^-T
+// terms is within 1e-16 relative of F_m for every m <= L (the missing part is
+// e^-T (2T)^(L-1) / ((2L-1)!! F_0): 8e-17 at L = 1, T = 40.5; 9e-17 at L = 4,
+// T = 48; 8e-17 at L = 8, T = 58).
+__host__ __device__ constexpr double far_T(int L) { return 38.0 + 2.5 * L; }
+// Unroll factor of the grouped kernel's far loop over bra primitives.
+__host__ __device__ constexpr int far_unroll(int la, int lb, int lc, int ld) {
+  return ncart(la) * ncart(lb) * ncart(lc) * ncart(ld) <= 9 ? 2 : 1;
+}
+// Warps per block of the grouped kernel: one block per SM, so that its warps
+// share one staged Boys slice and L1 keeps the rest of the SM's memory.
+__host__ __device__ constexpr int group_warps(int la, int lb, int lc, int ld) {
+  const int n = ncart(la) * ncart(lb) * ncart(lc) * ncart(ld);
+    return n == 1 ? 24 : n <= 9 ? 16 : n == 18 ? 12 : 8;
+}
 enum Mode { kStorePacked = 0, kJkRhf = 1, kJkUhf = 2, kSchwarz = 3, kBlock = 4 };
 
 // Density screening and precision of a J/K launch.  kScreenNone: every
@@ -100,8 +119,14 @@ enum Screen { kScreenNone = 0, kScreenFp64 = 1, kScreenMixed = 2 };
 // bAB = b(A-B) and K = N_a c_a N_b c_b exp(-ab/zeta |AB|^2) sqrt(2) pi^(5/4) / zeta,
 // so that the quartet prefactor 2 pi^(5/2) / (zeta eta sqrt(zeta+eta))
 // exp(...) of GaussianTwoElectrons.cpp:44-45 is K_ab K_cd / sqrt(zeta+eta).
-struct __align__(16) PrimPair {
-  double zeta, Px, Py, Pz, PAx, PAy, PAz, bABx, bABy, bABz, K, inv_zeta;
+// Kf = K (pi^(1/4) / sqrt 2) / sqrt(zeta) is the prefactor of far quartets
+// (eri_group.cuh).  128 B: one cache line per primitive pair, in the order of
+// use, so that an s-s pair reads two of its sectors.
+struct __align__(128) PrimPair {
+  double Px, Py, Pz, zeta;
+  double K, Kf, inv_zeta, PAx;
+  double PAy, PAz, bABx, bABy;
+  double bABz, pad[3];
 };
 // FP32 copy of a PrimPair for the mixed-precision kernels (48 B)
 struct __align__(16) PrimPairF {
@@ -157,6 +182,43 @@ struct __align__(16) Task {
   int lg = 0;
 };
 
+// The same 16 bytes as the grouped kernel (eri_group.cuh) reads them: nbra
+// consecutive bras of its bra list from bra_start (all with one first shell),
+// nket kets from ket_start, 2^lg lanes per ket, and per bra a pair of ket
+// masks from mask_off on: x = quartets of the build, y = those of them with a
+// primitive quartet that is not far.
+struct GroupTask {
+  int bra_start, ket_start, nket, nbra, lg;
+  unsigned mask_off;
+};
+constexpr int kGroupMaxBras = 16;
+// primitive quartets per lane a grouped task is kept below
+constexpr int kGroupTaskSteps = 256;
+// Tasks of a class (one bra, up to 32 kets) per SM from which its plain J/K
+// builds run the grouped kernel, whose blocks fill an SM each; twice as many on
+// concurrent class streams, where below it the one-bra-per-task kernel, whose
+// small blocks share the SMs with the other classes, is as fast or faster.  With
+// every class grouped: (H2O)32 / 6-31G* (80,000 to 958,000 tasks a class) 25.5 ->
+// 22.1 ms one after another and 25.2 -> 22.1 on streams, (H2O)16 (14,000 to
+// 153,000) 6.26 -> 5.83 and 4.99 -> 4.88, C9H20 / 6-31+G** (23,000 to 211,000)
+// 8.79 -> 8.55 but 6.94 -> 7.30, UHF C10H22 / 6-31G* (below 100,000) 5.03 -> 4.91
+// but 3.23 -> 3.57.
+constexpr int kGroupMinTasks = 750;
+
+// Ket primitive pairs by list position: block `pos >> 5` of a pair class's list
+// starts at record off[pos >> 5], record ik of it holds primitive pair ik of
+// its 32 pairs, field by field (kKetFields x 32 doubles), so that a warp's
+// lanes read a field of 32 neighbouring kets as one row.
+enum KetField { kKetPx = 0, kKetKf = 3, kKetInvZeta = 4, kKetBAB = 5, kKetZeta = 8, kKetK = 9, kKetFields = 10 };
+constexpr int kKetStride = kKetFields * 32;
+__host__ __device__ __forceinline__ Task pack_group_task(int bra_start, int ket_start, int nket, int nbra, int lg,
+                                                         unsigned mask_off) {
+  return Task{bra_start, ket_start, (int)mask_off, lg | nket << 8 | nbra << 16};
+}
+__host__ __device__ __forceinline__ GroupTask group_task(const Task &t) {
+  return GroupTask{t.bra_pos, t.ket_start, (t.lg >> 8) & 0xff, (t.lg >> 16) & 0xff, t.lg & 0xff, (unsigned)t.ket_end};
+}
+
 struct ClassLaunch {
   const int *bra_list;   // pair indices of the bra class, sorted by Q desc
   const int *ket_list;   // pair indices of the ket class, sorted by Q desc
@@ -164,6 +226,9 @@ struct ClassLaunch {
   int ntasks;            // tasks of this launch (of this shard)
   int task_offset;       // shard: launch task t is tasks[task_offset + t * task_stride]
   int task_stride;
+  const uint2 *masks;    // grouped launches: ket masks of the tasks
+  const double *ket_blocks;  // grouped launches: ket primitive pairs (KetField)
+  const int *ket_block_off;
   int same_class;        // bra class == ket class
   double threshold;
   // outputs by mode
@@ -264,6 +329,34 @@ __device__ __forceinline__ double exp_neg_far(double T) {
   return (double)exp2f((float)(y - n)) * __hiloint2double((ni + 1023) << 20, 0);
 }
 
+// A class's Boys slice, staged in shared memory (swizzled rows) or as the
+// per-order rows in global memory (plain rows of 64 bytes: four 16-byte loads).
+struct BoysShared {
+  const double *p;
+  __device__ __forceinline__ void row(int i, double *c) const {
+    const double2 *t = reinterpret_cast<const double2 *>(p + i * kBoysRow);
+    const int sw = (i >> 1) & 3;
+#pragma unroll
+    for (int j = 0; j < kBoysRow / 2; ++j) {
+      const double2 x = t[j ^ sw];
+      c[2 * j] = x.x;
+      c[2 * j + 1] = x.y;
+    }
+  }
+};
+struct BoysGlobal {
+  const double *p;
+  __device__ __forceinline__ void row(int i, double *c) const {
+    const double2 *t = reinterpret_cast<const double2 *>(p + i * kBoysRow);
+#pragma unroll
+    for (int k = 0; k < kBoysRow / 2; ++k) {
+      const double2 x = __ldg(t + k);
+      c[2 * k] = x.x;
+      c[2 * k + 1] = x.y;
+    }
+  }
+};
+
 // Boys function F_0..F_M at T.  Below kBoysTmax: 7-term Taylor expansion of
 // F_M about the nearest grid point, F_M(T) = sum_k F_{M+k}(T_i) (-dT)^k / k!,
 // from the shared-memory slice tab[i][k] = F_{M+k}(T_i)/k! (k < 7), then the
@@ -274,26 +367,27 @@ __device__ __forceinline__ double exp_neg_far(double T) {
 // Above: F_0 = sqrt(pi/T)/2 (erfc(sqrt T) < 3e-17 there) and the upward
 // recursion F_{m+1} = ((2m+1) F_m - e^-T) / (2T), 1/T as rsqrt(T)^2 and e^-T
 // from exp_neg_far.  The scale folds the quartet prefactor into every order.
-template <int M, class R>
-__device__ __forceinline__ void boys_eval(R *F, double T, double scale, const double *__restrict__ tab) {
+// e^-T is left out from far_T(M) on, where it is below the rounding of F_m.
+template <int M, class R, class Tab>
+__device__ __forceinline__ void boys_eval(R *F, double T, double scale, const Tab tab) {
   if (T < kBoysTmax) {
     const BoysGridPoint gp = boys_grid_point(T);
     const int i = gp.i;
     const double dt = gp.dt;  // -(T - T_i)
-    const double *t = tab + i * kBoysRow;
-    const int sw = (i >> 1) & 7;
+    double t[kBoysRow];
+    tab.row(i, t);
     // both polynomials in Estrin's scheme (pairs, then powers dt^2 and dt^4):
     // three dependent multiply-adds instead of six and seven in Horner's
     const double d2 = dt * dt, d4 = d2 * d2;
-    const double p01 = fma(t[1 ^ sw], dt, t[0 ^ sw]), p23 = fma(t[3 ^ sw], dt, t[2 ^ sw]);
-    const double p45 = fma(t[5 ^ sw], dt, t[4 ^ sw]);
+    const double p01 = fma(t[1], dt, t[0]), p23 = fma(t[3], dt, t[2]);
+    const double p45 = fma(t[5], dt, t[4]);
     double fm[M + 1];
-    fm[M] = fma(fma(t[6 ^ sw], d2, p45), d4, fma(p23, d2, p01));
+    fm[M] = fma(fma(t[6], d2, p45), d4, fma(p23, d2, p01));
     if (M > 0) {
       const double a01 = 1.0 + dt, a23 = fma(dt, 1.0 / 6.0, 0.5);
       const double a45 = fma(dt, 1.0 / 120.0, 1.0 / 24.0), a67 = fma(dt, 1.0 / 5040.0, 1.0 / 720.0);
       const double x = fma(fma(a67, d2, a45), d4, fma(a23, d2, a01));
-      const double e = t[7 ^ sw] * x;
+      const double e = t[7] * x;
       const double t2 = 2.0 * T;
 #pragma unroll
       for (int m = M - 1; m >= 0; --m) fm[m] = fma(t2, fm[m + 1], e) * (1.0 / (2 * m + 1));
@@ -305,7 +399,7 @@ __device__ __forceinline__ void boys_eval(R *F, double T, double scale, const do
     double f = 0.88622692545275801365 * r;  // sqrt(pi)/2 / sqrt(T)
     F[0] = (R)(f * scale);
     if (M > 0) {
-      const double e = exp_neg_far(T);
+      const double e = T < far_T(M) ? exp_neg_far(T) : 0.0;
       const double h = 0.5 * r * r;
 #pragma unroll
       for (int m = 0; m < M; ++m) {

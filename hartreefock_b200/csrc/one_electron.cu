@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(32 * kOneWarps) one_electron_kernel(const OneS
   constexpr int NA = ncart(LA), NB = ncart(LB), LT = LA + LB;
   using Cls = EriClass<LA, LB, 0, 0, false>;
   constexpr int NE = Cls::kAcc;
-  __shared__ double tab[kBoysGrid * kBoysRow];
+  __shared__ __align__(16) double tab[kBoysGrid * kBoysRow];
   stage_boys<LT>(tab, boys);
   const int lane = threadIdx.x & 31;
   for (int w = blockIdx.x * kOneWarps + (threadIdx.x >> 5); w < npairs; w += gridDim.x * kOneWarps) {
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(32 * kOneWarps) one_electron_kernel(const OneS
       }
       const double Tb = p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
       double F[LT + 1];
-      boys_eval<LT, double>(F, Tb, -nuc[4 * c + 3] * 2.0 * M_PI * ip * cc, tab);
+      boys_eval<LT>(F, Tb, -nuc[4 * c + 3] * 2.0 * M_PI * ip * cc, BoysShared{tab});
       Cls::template prim<double>(accE, F, PA[0], PA[1], PA[2], -PC[0], -PC[1], -PC[2], 0.5 * ip, 1.0, 0.0, 0.0, 0.0,
                                  0.0, 0.0);
     }
