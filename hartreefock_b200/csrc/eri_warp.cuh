@@ -11,11 +11,14 @@
 //      intermediates in shared memory, and add the [e0|f0] entries they own
 //      to register accumulators (the contraction);
 //   2. the contracted [e0|f0] block goes to shared memory and the lanes
-//      expand bra rows (a b) of the (ab|cd) block with the row-wise
-//      horizontal recursion (EriRows), normalised, into a shared block;
+//      expand it into the normalised (ab|cd) block there, element by element
+//      with the horizontal recursions as tables (HrrTable): every lane runs the
+//      same code.  (A row (a b) per lane ran the generated row code, a switch
+//      over the rows, one lane at a time.);
 //   3. the lanes digest the block: every element of J_ab, J_cd, K_ac, K_ad,
 //      K_bc, K_bd is one lane's dot product over the block, then one atomic
-//      (or the packed-table store).
+//      (or the packed-table store).  The density entries are read side by side
+//      into shared memory first.
 //
 // Work units are single quartets: unit u of a launch is ket u % 32 of task
 // u / 32 (units past a task's last ket are skipped), walked grid-stride by
@@ -80,6 +83,8 @@ __device__ __forceinline__ void boys_global(double *F, double T, double scale, c
 // Shared-memory footprint of one warp, in bytes: the program's slots and the
 // contracted block(s) in R, the normalised (ab|cd) block in FP64 with rows
 // padded to an odd length (conflict-free column reads).
+constexpr int kHrrMonomials = 11;  // monomials of HrrTable's terms
+
 template <int LA, int LB, int LC, int LD, bool REF>
 struct WarpShape {
   using P = WarpProg<LA, LB, LC, LD, REF>;
@@ -177,16 +182,57 @@ __device__ __forceinline__ void warp_contract(const EngineView &v, int bp, int k
   __syncwarp();
 }
 
+// One term list of HrrTable over vals[e * stride]: sum of coefficient x
+// monomial x value in the table's order.
+template <int TERMS, class R>
+__device__ __forceinline__ R hrr_sum(const uint2 t, const R *mono, const R *vals, int stride) {
+  R s = R(0);
+#pragma unroll
+  for (int k = 0; k < TERMS; ++k) {
+    const unsigned w = ((k & 2 ? t.y : t.x) >> (16 * (k & 1))) & 0xffffu;
+    R c = mono[(w >> 8) & 15u];
+    if (w & 0x1000u) c += c;
+    const R x = vals[(w & 0xffu) * stride];
+    s = k == 0 ? c * x : s + c * x;
+  }
+  return s;
+}
+
+// (ab|cd) from a contracted [e0|f0] block in shared memory, bra components of
+// one a at a time: the bra recursion into tmp[b][f], then the ket recursion;
+// write(ab, cd, value).  bra / ket: the monomials of A - B and C - D.
+template <int LA, int LB, int LC, int LD, class R, class W>
+__device__ __forceinline__ void warp_expand(const R *acc, const R *bra, const R *ket, R *tmp, W write) {
+  constexpr int NA = ncart(LA), NB = ncart(LB), NCD = ncart(LC) * ncart(LD);
+  constexpr int NF = WarpProg<LA, LB, LC, LD, false>::kNf;
+  using Bra = HrrTable<LA, LB>;
+  using Ket = HrrTable<LC, LD>;
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int a = 0; a < NA; ++a) {
+#pragma unroll 1
+    for (int x = lane; x < NB * NF; x += 32) {
+      const int b = x / NF;
+      tmp[x] = hrr_sum<Bra::kTerms, R>(__ldg(Bra::rows() + a * NB + b), bra, acc + (x - b * NF), NF);
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int x = lane; x < NB * NCD; x += 32) {
+      const int b = x / NCD, cd = x - b * NCD;
+      write(a * NB + b, cd, hrr_sum<Ket::kTerms, R>(__ldg(Ket::rows() + cd), ket, tmp + b * NF, 1));
+    }
+    __syncwarp();
+  }
+}
+
 // The normalised (ab|cd) block of the quartet into o[ab * NCDP + cd] (FP64),
 // with the reference's per-element bra/ket orientation for its (dd|dd)
 // convention (see dddd_reference_values).
 template <int LA, int LB, int LC, int LD, bool REF, class R>
 __device__ __forceinline__ void warp_block(const EngineView &v, int bp, int kp, R *w, R *acc_sh, double *o) {
   using S = WarpShape<LA, LB, LC, LD, REF>;
-  constexpr int NB = S::NB, NC = S::NC, ND = S::ND, NCD = S::NCD, NCDP = S::NCDP;
+  constexpr int NB = S::NB, ND = S::ND, NCDP = S::NCDP;
   const int lane = threadIdx.x & 31;
-  const R X0 = R(v.pair_AB[3 * bp]), X1 = R(v.pair_AB[3 * bp + 1]), X2 = R(v.pair_AB[3 * bp + 2]);
-  const R Y0 = R(v.pair_AB[3 * kp]), Y1 = R(v.pair_AB[3 * kp + 1]), Y2 = R(v.pair_AB[3 * kp + 2]);
   int mode = 0;  // 0: (bp|kp) only, 1: (kp|bp) only, 2: both, chosen per element
   if constexpr (S::kOrient) {
     const int sab = v.pair_sa[bp], skt = v.pair_sa[kp];
@@ -197,41 +243,38 @@ __device__ __forceinline__ void warp_block(const EngineView &v, int bp, int kp, 
   if constexpr (S::kOrient) {
     if (mode != 0) warp_contract<LA, LB, LC, LD, REF, R>(v, kp, bp, w, acc_r);
   }
-  const int aoa = v.pair_ao_a[bp], aob = v.pair_ao_b[bp], aoc = v.pair_ao_a[kp], aod = v.pair_ao_b[kp];
-  const bool bdiag = v.pair_sa[bp] == v.pair_sb[bp], kdiag = v.pair_sa[kp] == v.pair_sb[kp];
-  for (int ab = lane; ab < S::NAB; ab += 32) {
-    const int a = ab / NB, b = ab - a * NB;
-    R out[NCD];
-    if (mode == 1) {
-      if constexpr (S::kOrient)
-        EriRows<LA, LB, LC, LD>::template col<R>(out, ab, acc_r, 1, Y0, Y1, Y2, X0, X1, X2);
-    } else {
-      EriRows<LA, LB, LC, LD>::template row<R>(out, ab, acc_f, 1, X0, X1, X2, Y0, Y1, Y2);
-    }
-    if constexpr (S::kOrient) {
-      if (mode == 2) {
-        R sw[NCD];
-        EriRows<LA, LB, LC, LD>::template col<R>(sw, ab, acc_r, 1, Y0, Y1, Y2, X0, X1, X2);
-        const int I = aoa + a, J = aob + b;
-        const int o1 = bdiag ? max(I, J) : I, o2 = bdiag ? min(I, J) : J;
-#pragma unroll
-        for (int c = 0; c < NC; ++c)
-#pragma unroll
-          for (int d = 0; d < ND; ++d) {
-            const int K = aoc + c, L = aod + d;
-            const int o3 = kdiag ? max(K, L) : K, o4 = kdiag ? min(K, L) : L;
-            if (!(o1 > o3 || (o1 == o3 && o2 >= o4))) out[c * ND + d] = sw[c * ND + d];
-          }
-      }
-    }
-    const double nab = comp_norm<LA>(a) * comp_norm<LB>(b);
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-      for (int d = 0; d < ND; ++d)
-        o[ab * NCDP + c * ND + d] = double(out[c * ND + d]) * (nab * comp_norm<LC>(c) * comp_norm<LD>(d));
+  // monomials of A - B and C - D, where the recursions' slots were
+  static_assert(2 * kHrrMonomials + NB * WarpProg<LA, LB, LC, LD, REF>::kNf <= S::kWork, "expansion fits the slots");
+  R *bra = w, *ket = w + kHrrMonomials, *tmp = w + 2 * kHrrMonomials;
+  if (lane < 2 * kHrrMonomials) {
+    const int m = lane < kHrrMonomials ? lane : lane - kHrrMonomials;
+    const double *AB = v.pair_AB + 3 * (lane < kHrrMonomials ? bp : kp);
+    const R x = R(AB[0]), y = R(AB[1]), z = R(AB[2]);
+    const R p = m == 1 || (m >= 4 && m <= 6) ? x : m == 2 || m == 7 || m == 8 ? y : z;
+    const R q = m == 4 ? x : m == 5 || m == 7 ? y : z;
+    w[lane] = m == 0 ? R(1) : m <= 3 ? p : m <= 9 ? p * q : R(0);
   }
   __syncwarp();
+  const auto norm = [](int ab, int cd) {
+    return comp_norm<LA>(ab / NB) * comp_norm<LB>(ab % NB) * comp_norm<LC>(cd / ND) * comp_norm<LD>(cd % ND);
+  };
+  if (mode != 1)
+    warp_expand<LA, LB, LC, LD, R>(acc_f, bra, ket, tmp, [&](int ab, int cd, R x) { o[ab * NCDP + cd] = double(x) * norm(ab, cd); });
+  if constexpr (S::kOrient) {
+    // the swapped block's bra is (c d)
+    if (mode == 1)
+      warp_expand<LC, LD, LA, LB, R>(acc_r, ket, bra, tmp, [&](int cd, int ab, R x) { o[ab * NCDP + cd] = double(x) * norm(ab, cd); });
+    if (mode == 2) {
+      const int aoa = v.pair_ao_a[bp], aob = v.pair_ao_b[bp], aoc = v.pair_ao_a[kp], aod = v.pair_ao_b[kp];
+      const bool bdiag = v.pair_sa[bp] == v.pair_sb[bp], kdiag = v.pair_sa[kp] == v.pair_sb[kp];
+      warp_expand<LC, LD, LA, LB, R>(acc_r, ket, bra, tmp, [&](int cd, int ab, R x) {
+        const int I = aoa + ab / NB, J = aob + ab % NB, K = aoc + cd / ND, L = aod + cd % ND;
+        const int o1 = bdiag ? max(I, J) : I, o2 = bdiag ? min(I, J) : J;
+        const int o3 = kdiag ? max(K, L) : K, o4 = kdiag ? min(K, L) : L;
+        if (!(o1 > o3 || (o1 == o3 && o2 >= o4))) o[ab * NCDP + cd] = double(x) * norm(ab, cd);
+      });
+    }
+  }
 }
 
 template <int LA, int LB, int LC, int LD, int MODE, bool REF, int SCR>
@@ -293,56 +336,75 @@ __global__ void __launch_bounds__(32 * WarpShape<LA, LB, LC, LD, REF>::kWarps)
       double *Jm = cl.J + mv.base, *Kam = cl.Ka + mv.base, *Kbm = kUhf ? cl.Kb + mv.base : nullptr;
       constexpr int nK = NA * NC + NA * ND + NB * NC + NB * ND;
       constexpr int total = NAB + NCD + nK * (kUhf ? 2 : 1);
+      static_assert(total <= S::kRDoubles, "density entries fit the work area");
+      // element x of J_ab, J_cd, then per spin K_ac, K_ad, K_bc, K_bd: its
+      // matrix offset (and so that of the density entry of the same indices)
+      const auto at = [&](int x) {
+        int r, c;
+        if (x < NAB) {
+          r = aoa + x / NB, c = aob + x % NB;
+        } else if ((x -= NAB) < NCD) {
+          r = aoc + x / ND, c = aod + x % ND;
+        } else {
+          x -= NCD;
+          if (kUhf && x >= nK) x -= nK;
+          if (x < NA * NC) {
+            r = aoa + x / NC, c = aoc + x % NC;
+          } else if ((x -= NA * NC) < NA * ND) {
+            r = aoa + x / ND, c = aod + x % ND;
+          } else if ((x -= NA * ND) < NB * NC) {
+            r = aob + x / NC, c = aoc + x % NC;
+          } else {
+            x -= NB * NC;
+            r = aob + x / ND, c = aod + x % ND;
+          }
+        }
+        return r * n + c;
+      };
+      double *D = base;  // the density entries, in the same order
+      for (int x = lane; x < total; x += 32)
+        D[x] = __ldg((x < NAB + NCD ? DJ : kUhf && x >= NAB + NCD + nK ? Db : Da) + at(x));
+      __syncwarp();
       for (int x = lane; x < total; x += 32) {
         double t = 0.0;
         if (x < NAB) {
-          const int a = x / NB, b = x - a * NB;
 #pragma unroll 4
-          for (int cd = 0; cd < NCD; ++cd) {
-            const int c = cd / ND, d = cd - c * ND;
-            t += o[x * NCDP + cd] * __ldg(&DJ[(aoc + c) * n + aod + d]);
-          }
-          atomicAdd(&Jm[(aoa + a) * n + aob + b], 2.0 * s * t);
+          for (int cd = 0; cd < NCD; ++cd) t += o[x * NCDP + cd] * D[NAB + cd];
+          atomicAdd(&Jm[at(x)], 2.0 * s * t);
         } else if (x < NAB + NCD) {
-          const int cd = x - NAB, c = cd / ND, d = cd - c * ND;
+          const int cd = x - NAB;
 #pragma unroll 4
-          for (int ab = 0; ab < NAB; ++ab) {
-            const int a = ab / NB, b = ab - a * NB;
-            t += o[ab * NCDP + cd] * __ldg(&DJ[(aoa + a) * n + aob + b]);
-          }
-          atomicAdd(&Jm[(aoc + c) * n + aod + d], 2.0 * s * t);
+          for (int ab = 0; ab < NAB; ++ab) t += o[ab * NCDP + cd] * D[ab];
+          atomicAdd(&Jm[at(x)], 2.0 * s * t);
         } else {
           int y = x - NAB - NCD;
           const bool beta = kUhf && y >= nK;
           if (beta) y -= nK;
-          const double *D = beta ? Db : Da;
-          double *Km = beta ? Kbm : Kam;
+          const double *Dac = D + NAB + NCD + (beta ? nK : 0), *Dad = Dac + NA * NC, *Dbc = Dad + NA * ND,
+                       *Dbd = Dbc + NB * NC;
           if (y < NA * NC) {  // K_ac = sum_bd (ab|cd) D_bd
             const int a = y / NC, c = y - a * NC;
             for (int b = 0; b < NB; ++b)
 #pragma unroll
-              for (int d = 0; d < ND; ++d) t += o[(a * NB + b) * NCDP + c * ND + d] * __ldg(&D[(aob + b) * n + aod + d]);
-            atomicAdd(&Km[(aoa + a) * n + aoc + c], s * t);
+              for (int d = 0; d < ND; ++d) t += o[(a * NB + b) * NCDP + c * ND + d] * Dbd[b * ND + d];
           } else if ((y -= NA * NC) < NA * ND) {  // K_ad = sum_bc (ab|cd) D_bc
             const int a = y / ND, d = y - a * ND;
             for (int b = 0; b < NB; ++b)
 #pragma unroll
-              for (int c = 0; c < NC; ++c) t += o[(a * NB + b) * NCDP + c * ND + d] * __ldg(&D[(aob + b) * n + aoc + c]);
-            atomicAdd(&Km[(aoa + a) * n + aod + d], s * t);
+              for (int c = 0; c < NC; ++c) t += o[(a * NB + b) * NCDP + c * ND + d] * Dbc[b * NC + c];
           } else if ((y -= NA * ND) < NB * NC) {  // K_bc = sum_ad (ab|cd) D_ad
             const int b = y / NC, c = y - b * NC;
             for (int a = 0; a < NA; ++a)
 #pragma unroll
-              for (int d = 0; d < ND; ++d) t += o[(a * NB + b) * NCDP + c * ND + d] * __ldg(&D[(aoa + a) * n + aod + d]);
-            atomicAdd(&Km[(aob + b) * n + aoc + c], s * t);
+              for (int d = 0; d < ND; ++d) t += o[(a * NB + b) * NCDP + c * ND + d] * Dad[a * ND + d];
           } else {  // K_bd = sum_ac (ab|cd) D_ac
             y -= NB * NC;
             const int b = y / ND, d = y - b * ND;
             for (int a = 0; a < NA; ++a)
 #pragma unroll
-              for (int c = 0; c < NC; ++c) t += o[(a * NB + b) * NCDP + c * ND + d] * __ldg(&D[(aoa + a) * n + aoc + c]);
-            atomicAdd(&Km[(aob + b) * n + aod + d], s * t);
+              for (int c = 0; c < NC; ++c) t += o[(a * NB + b) * NCDP + c * ND + d] * Dac[a * NC + c];
           }
+          atomicAdd(&(beta ? Kbm : Kam)[at(x)], s * t);
         }
       }
     }

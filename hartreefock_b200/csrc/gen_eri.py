@@ -804,6 +804,28 @@ class WarpProgram:
         return dict(ops=ops, bounds=bounds, nslots=nslots, fslots=fslots, acc=acc, ne=len(E), nf=len(Fc))
 
 
+def hrr_table(la, lb):
+    """The horizontal recursion of a pair as data for the warp kernel: per
+    component (a b) four 16-bit terms, element e of [e0| in bits 0-7, monomial
+    of A-B in bits 8-11 (0: 1, 1-3: x y z, 4-9: xx xy xz yy yz zz, 10: zero, for
+    unused terms), bit 12: coefficient 2."""
+    E = comps_range(la, la + lb)
+    mono = {(0, 0, 0): 0, (1, 0, 0): 1, (0, 1, 0): 2, (0, 0, 1): 3, (2, 0, 0): 4, (1, 1, 0): 5, (1, 0, 1): 6,
+            (0, 2, 0): 7, (0, 1, 1): 8, (0, 0, 2): 9}
+    rows, memo = [], {}
+    for a in comps(la):
+        for b in comps(lb):
+            terms = []
+            for e, poly in sorted(hrr_expansion(a, b, memo).items(), key=lambda kv: E.index(kv[0])):
+                (m, c), = poly.items()
+                assert c in (1, 2)
+                terms.append(E.index(e) | mono[m] << 8 | (c - 1) << 12)
+            assert len(terms) <= (1, 2, 4)[lb]
+            terms += [10 << 8] * (4 - len(terms))
+            rows.append((terms[0] | terms[1] << 16, terms[2] | terms[3] << 16))
+    return rows
+
+
 def warp_flops(prog):
     """flops of one primitive quartet's recursions as the generated straight-line code counts them"""
     return None
@@ -816,7 +838,19 @@ def emit_warp(out_dir):
     serves)."""
     pairs, quartets = canonical_classes()
     hdr = ["// Generated by gen_eri.py -- do not edit.", "#pragma once", "", "#include <stdint.h>", "",
-           "namespace hfg {", "", "template <int LA, int LB, int LC, int LD, bool REF> struct WarpProg;"]
+           "namespace hfg {", "", "template <int LA, int LB, int LC, int LD, bool REF> struct WarpProg;",
+           "// horizontal recursion terms of a pair's components (hrr_table)",
+           "template <int LA, int LB> struct HrrTable;"]
+    for (la, lb) in pairs:
+        rows = hrr_table(la, lb)
+        hdr.append(f"static __device__ const uint2 kHrrTable_{la}{lb}[] = {{")
+        for k in range(0, len(rows), 4):
+            hdr.append("    " + ", ".join("{%du, %du}" % r for r in rows[k:k + 4]) + ",")
+        hdr.append("};")
+        hdr.append(f"template <> struct HrrTable<{la}, {lb}> {{")
+        hdr.append(f"  static constexpr int kTerms = {(1, 2, 4)[lb]};")
+        hdr.append(f"  static __device__ __forceinline__ const uint2 *rows() {{ return kHrrTable_{la}{lb}; }}")
+        hdr.append("};")
     for (la, lb, lc, ld) in quartets:
         if not is_split_class(la, lb, lc, ld):
             continue
@@ -844,6 +878,7 @@ def emit_warp(out_dir):
             hdr.append(f"  static constexpr int kOps = {len(pr['ops'])};")
             hdr.append(f"  static constexpr int kLevels = {len(pr['bounds']) - 1};")
             hdr.append(f"  static constexpr int kAcc = {pr['ne'] * pr['nf']};")
+            hdr.append(f"  static constexpr int kNf = {pr['nf']};")
             hdr.append("  static __device__ __forceinline__ const uint4 *ops() { return kWarpOps_%s; }" % tag)
             hdr.append("  static __device__ __forceinline__ const uint16_t *acc() { return kWarpAcc_%s; }" % tag)
             hdr.append("  static __device__ __forceinline__ int bound(int l) {")
