@@ -183,9 +183,11 @@ struct hfg_ctx {
   bool use_graphs = false;
   bool use_streams = false;  // class kernels over the auxiliary streams (hfg_set_streams)
   // large classes with both kernels: 1 = the warp-cooperative kernel, 0 =
-  // the split path (primitive kernel + HRR/digest over scratch); per class,
-  // from hfg_autotune_paths / hfg_set_class_path, else the default below
+  // the split path (primitive kernel + HRR/digest over scratch), -1 = by the
+  // class's primitive quartets (warp_prim_limit); per class, set by
+  // hfg_autotune_paths / hfg_set_class_path
   int8_t warp_class[kNumClasses] = {};
+  int64_t class_prims[kNumClasses] = {};  // primitive quartets of each class's tasks
   // direct builds: the fused and warp-cooperative class kernels take their
   // tasks from a device work queue (one counter per class, one atomic per
   // warp and task) instead of a grid-stride walk
@@ -325,7 +327,16 @@ struct hfg_ctx {
 
 // the large class runs on the warp-cooperative kernel (classes with only
 // that kernel always do)
-static bool class_on_warp(const hfg_ctx *c, int cls) { return kWarp[cls] && (c->warp_class[cls] || !kSplit[cls]); }
+// (prec: the launch's form, see ClassLauncher; a mixed one chooses FP64 or FP32
+// per quartet there and per task on the split path, and keeps to the latter
+// but for (dd|dd))
+static bool class_on_warp(const hfg_ctx *c, int cls, int prec) {
+  if (!kWarp[cls] || !kSplit[cls]) return kWarp[cls] != nullptr;
+  if (c->warp_class[cls] >= 0) return c->warp_class[cls] != 0;
+  const ClassEntry &e = kClasses[cls];
+  if (prec == 2) return e.la + e.lb + e.lc + e.ld == 8;
+  return c->class_prims[cls] <= warp_prim_limit(e.la, e.lb, e.lc, e.ld);
+}
 
 namespace hfg {
 
@@ -437,6 +448,7 @@ static void build_group_tasks(const hfg_ctx *c, QuartetClass &q, const std::vect
 // bra's position in the concatenated bucket list.
 static void build_quartet_classes(hfg_ctx *c, double threshold) {
   c->qclasses.clear();
+  std::fill(std::begin(c->class_prims), std::end(c->class_prims), int64_t(0));
   for (int ci = 0; ci < kNumClasses; ++ci) {
     const ClassEntry &ce = kClasses[ci];
     QuartetClass q;
@@ -531,6 +543,7 @@ static void build_quartet_classes(hfg_ctx *c, double threshold) {
     q.flops = (double)q.prim_quartets * (pf + boys_geom_flops(ltot)) + (double)q.shell_quartets * hf;
     if (kGroup[ci] && (int64_t)q.tasks.size() >= (int64_t)c->group_min_tasks * c->num_sms)
       build_group_tasks(c, q, ends, segmax, kprim, target, pf + boys_geom_flops(ltot), hf);
+    c->class_prims[ci] = q.prim_quartets;
     if (!q.tasks.empty()) c->qclasses.push_back(std::move(q));
   }
   // largest classes first
@@ -773,7 +786,7 @@ static int ncomp_range(int lo, int hi) {
 static void split_chunking(const hfg_ctx *c, int cls, int ntasks, bool ref, size_t *need, int *chunk_tasks);
 static int scratch_regions(const hfg_ctx *c);
 // the class runs the split (primitive + HRR/digest) kernels over scratch
-static bool uses_split(const hfg_ctx *c, int cls) { return kSplit[cls] && !class_on_warp(c, cls); }
+static bool uses_split(const hfg_ctx *c, int cls, int prec) { return kSplit[cls] && !class_on_warp(c, cls, prec); }
 static hfg_status grow_scratch(hfg_ctx *c, int slot, size_t need);
 
 struct ClassStreams {
@@ -801,12 +814,12 @@ struct ClassStreams {
   // Sizes the scratch region of every split class before anything of the
   // build is launched, following the order pick() will hand out regions in
   // (`ntasks` per quartet class, in class order).
-  hfg_status presize(const std::vector<int> &ntasks, bool ref) {
+  hfg_status presize(const std::vector<int> &ntasks, bool ref, int prec) {
     std::vector<size_t> need(hfg_ctx::kAux, 0);
     int k = 0;
     for (size_t i = 0; i < c->qclasses.size(); ++i) {
       const int cls = c->qclasses[i].cls;
-      if (!uses_split(c, cls) || ntasks[i] <= 0) continue;
+      if (!uses_split(c, cls, prec) || ntasks[i] <= 0) continue;
       size_t nd = 0;
       int chunk = 1;
       split_chunking(c, cls, ntasks[i], ref, &nd, &chunk);
@@ -876,7 +889,7 @@ static hfg_status launch_class(hfg_ctx *c, const QuartetClass &q, const ClassLau
     ++*launches;
     return HFG_OK;
   }
-  if (class_on_warp(c, q.cls) && mode != kBlock) {
+  if (class_on_warp(c, q.cls, prec) && mode != kBlock) {
     kWarp[q.cls](c->view(), cl, mode, ref, prec, 0, s);
     ++*launches;
     return HFG_OK;
@@ -918,6 +931,7 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
   if ((st = ensure(&c->d_J, nn)) != HFG_OK || (st = ensure(&c->d_Ka, nn)) != HFG_OK) return st;
   if (uhf && ((st = ensure(&c->d_Kb, nn)) != HFG_OK || (st = ensure(&c->d_Pt, nn)) != HFG_OK)) return st;
   const bool precise = c->precision_form();
+  const int prec = !precise ? 0 : c->mixed_cutoff > 0 ? 2 : 1;
   const bool incremental = precise && c->opts.incremental;
   const bool fresh = !c->inc_valid || c->inc_uhf != uhf;
   const int eg = std::max(1, std::min(1024, (int)((nn + 255) / 256)));
@@ -974,11 +988,10 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
   {
     std::vector<int> nt(c->qclasses.size());
     for (size_t i = 0; i < nt.size(); ++i) nt[i] = base_launch(c, c->qclasses[i], true).ntasks;
-    if ((st = cs.presize(nt, ref)) != HFG_OK) return st;
+    if ((st = cs.presize(nt, ref, prec)) != HFG_OK) return st;
   }
   if (!capturing) HFG_CUDA(cudaEventRecord(c->ev0, s));
   if ((st = cs.fork()) != HFG_OK) return st;
-  const int prec = !precise ? 0 : c->mixed_cutoff > 0 ? 2 : 1;
   c->stats = hfg_stats{};
   for (size_t qi = 0; qi < nq; ++qi) {
     QuartetClass &q = c->qclasses[qi];
@@ -994,10 +1007,10 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
     cl.mixed_cutoff = (float)c->mixed_cutoff;
     cl.counters = precise ? c->d_counters : nullptr;
     if (cl.ntasks > 0) {
-      const cudaStream_t cls_stream = cs.pick(uses_split(c, q.cls));
+      const cudaStream_t cls_stream = cs.pick(uses_split(c, q.cls, prec));
       ClassLaunch cll = cl;
-      if ((c->use_queue || compact || cl.masks) && !uses_split(c, q.cls)) cll.queue = c->d_queue + qi;
-      if (compact && !uses_split(c, q.cls)) {
+      if ((c->use_queue || compact || cl.masks) && !uses_split(c, q.cls, prec)) cll.queue = c->d_queue + qi;
+      if (compact && !uses_split(c, q.cls, prec)) {
         const int cg = std::max(1, std::min(c->num_sms * 8, (cl.ntasks + 7) / 8));
         compact_screened_tasks<<<cg, 256, 0, cls_stream>>>(c->view(), cl, c->d_task_active + c->task_base[qi],
                                                             c->d_task_counts + qi);
@@ -1234,7 +1247,7 @@ static hfg_status batch_build(hfg_ctx *c, bool uhf, const double *dPa, const dou
   {
     std::vector<int> nt(c->qclasses.size());
     for (size_t i = 0; i < nt.size(); ++i) nt[i] = compact ? counts[i] : base_launch(c, c->qclasses[i], true).ntasks;
-    if ((st = cs.presize(nt, ref)) != HFG_OK) return st;
+    if ((st = cs.presize(nt, ref, 0)) != HFG_OK) return st;
   }
   HFG_CUDA(cudaEventRecord(c->ev0, s));
   if ((st = cs.fork()) != HFG_OK) return st;
@@ -1256,7 +1269,7 @@ static hfg_status batch_build(hfg_ctx *c, bool uhf, const double *dPa, const dou
     cl.Ka = c->d_Ka;
     cl.Kb = c->d_Kb;
     if (cl.ntasks > 0) {
-      const cudaStream_t cls_stream = cs.pick(uses_split(c, q.cls));
+      const cudaStream_t cls_stream = cs.pick(uses_split(c, q.cls, 0));
       st = launch_class(c, q, cl, uhf ? kJkUhf : kJkRhf, ref, 0, cls_stream, &launches, cs.slot);
       if (st != HFG_OK) return st;
     }
@@ -1475,14 +1488,9 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
   if (const char *e = std::getenv("HFG_GROUP_MIN_TASKS")) ctx->group_min_tasks = std::max(0, std::atoi(e));
   // tuning: HFG_PRIM_TARGET sets the lane-group target (0: one lane per quartet)
   if (const char *e = std::getenv("HFG_PRIM_TARGET")) ctx->prim_target = std::max(0, std::atoi(e));
-  // default kernel per large class: the warp-cooperative kernel where one
-  // quartet's primitive work fills a warp -- (dd|dd), 1296 Cartesian
-  // components -- the split path for the rest; HFG_SPLIT_PATH=1 / HFG_WARP_PATH=1
-  // put every large class on one of them
-  for (int k = 0; k < kNumClasses; ++k) {
-    const ClassEntry &e = kClasses[k];
-    ctx->warp_class[k] = kWarp[k] && e.la + e.lb + e.lc + e.ld >= 8 ? 1 : 0;
-  }
+  // default kernel per large class: by its primitive quartets (warp_prim_limit);
+  // HFG_SPLIT_PATH=1 / HFG_WARP_PATH=1 put every large class on one of them
+  std::fill(std::begin(ctx->warp_class), std::end(ctx->warp_class), int8_t(-1));
   if (const char *e = std::getenv("HFG_WORK_QUEUE")) ctx->use_queue = std::atoi(e) != 0;
   if (const char *e = std::getenv("HFG_NO_COMPACT")) ctx->use_compaction = std::atoi(e) == 0;
   // tuning: HFG_SCRATCH_MB bounds the split path's scratch (all regions together)
@@ -2000,7 +2008,7 @@ hfg_status hfg_class_profile(const hfg_ctx *c, hfg_class_time *out, int32_t cap,
     const ClassEntry &e = kClasses[q.cls];
     out[n] = hfg_class_time{e.la,    e.lb,    e.lc,         e.ld, q.shell_quartets, q.function_quartets, q.prim_quartets,
                             q.flops, (double)q.last_ms, (int64_t)q.tasks.size(),
-                            q.warp_work > 0 ? q.lane_work / q.warp_work : 0.0, class_on_warp(c, q.cls) ? 1 : 0, 0};
+                            q.warp_work > 0 ? q.lane_work / q.warp_work : 0.0, class_on_warp(c, q.cls, c->mixed_cutoff > 0 ? 2 : 0) ? 1 : 0, 0};
     ++n;
   }
   *count = n;

@@ -102,6 +102,28 @@ __host__ __device__ constexpr int group_warps(int la, int lb, int lc, int ld) {
   const int n = ncart(la) * ncart(lb) * ncart(lc) * ncart(ld);
     return n == 1 ? 24 : n <= 9 ? 16 : n == 18 ? 12 : 8;
 }
+// Primitive quartets of a large class up to which its builds run the
+// warp-cooperative kernel, a quartet per warp, instead of the split path, a
+// quartet per thread: the thread takes 50 to 300 us over one quartet however
+// few there are, the warp a fraction of that, until there are enough to fill
+// the GPU with threads.  The lines are where the two meet (us per J/K build of
+// (H2O)2, 4, 8, 12, 16 / 6-31G*, warp kernel against split path): (dd|dp) 45, 45,
+// 66, 125, 273 against 286, 292, 315, 351, 432 (9,074 primitive quartets in the
+// last); (dd|pp) 50, 51, 95, 164, 271 against 111, 139, 130, 165, 172 (9,019 in
+// (H2O)12); (dd|ds) 39, 43, 93 against 59, 77, 87 (5,523 in (H2O)8); (dd|ps) 56, 54,
+// 156 against 52, 58, 69 (4,541 in (H2O)4); (dp|pp) 78, 109 against 94, 104 (3,994 in
+// (H2O)4); (dp|ds) is level at 470.  (dd|dd) is faster here at every size (0.24
+// against 0.82 ms at (H2O)16, before its recursions became tables).  (dp|dp) would
+// gain too (56 against 157 at (H2O)2), but its transfer in this kernel's
+// association is 3.1e-12 off on two cancelling elements of O2 / 6-31G* (1.3e-12 on
+// the split path), so it stays where it was.
+__host__ __device__ constexpr long long warp_prim_limit(int la, int lb, int lc, int ld) {
+  const int ket = 10 * lc + ld;
+  if (la == 2 && lb == 2)
+    return ket == 22 ? (1ll << 62) : ket == 21 ? 16000 : ket == 11 ? 9000 : ket == 20 ? 5000 : ket == 10 ? 4500 : 0;
+  return ket == 11 ? 2500 : 0;
+}
+
 enum Mode { kStorePacked = 0, kJkRhf = 1, kJkUhf = 2, kSchwarz = 3, kBlock = 4 };
 
 // Density screening and precision of a J/K launch.  kScreenNone: every
