@@ -31,6 +31,8 @@ static hfg_status fail(hfg_status st, const std::string &msg) {
 // hfg_one_electron)
 hfg_status fail_external(hfg_status st, const std::string &msg) { return fail(st, msg); }
 static const std::vector<double> &boys_table_host();
+void *ctx_handle(hfg_ctx *c);
+void ctx_keep_handle(hfg_ctx *c, void *h, void (*destroy)(void *));
 const std::vector<double> &boys_table_for_external() { return boys_table_host(); }
 
 #define HFG_CUDA(call)                                                                        \
@@ -252,6 +254,10 @@ struct hfg_ctx {
   int *d_task_counts = nullptr;
   int *d_queue = nullptr;  // per quartet class: the device work queue's counter
   std::vector<int> task_base;  // per quartet class, offset into d_task_active
+  // a library handle of another translation unit (the MO transform's cuBLAS
+  // handle), destroyed with the context
+  void *handle = nullptr;
+  void (*handle_destroy)(void *) = nullptr;
   hfg_stats stats{};
   bool profiling = false;
   bool precision_form() const { return opts.density_screening || opts.incremental || mixed_cutoff > 0; }
@@ -291,6 +297,7 @@ struct hfg_ctx {
     for (int i = 0; i < kAux; ++i)
       if (aux[i]) cudaStreamSynchronize(aux[i]);
     if (stream) cudaStreamSynchronize(stream);
+    if (handle) handle_destroy(handle);
     for (auto &q : qclasses) {
       cudaFree(q.d_tasks);
       cudaFree(q.d_gtasks);
@@ -324,6 +331,14 @@ struct hfg_ctx {
     if (stream) cudaStreamDestroy(stream);
   }
 };
+
+namespace hfg {
+void *ctx_handle(hfg_ctx *c) { return c->handle; }
+void ctx_keep_handle(hfg_ctx *c, void *h, void (*destroy)(void *)) {
+  c->handle = h;
+  c->handle_destroy = destroy;
+}
+}  // namespace hfg
 
 // the large class runs on the warp-cooperative kernel (classes with only
 // that kernel always do)

