@@ -6,6 +6,7 @@
 #include <cstring>
 #include <memory>
 #include <cstdlib>
+#include <future>
 #include <mutex>
 #include <numeric>
 #include <set>
@@ -254,12 +255,12 @@ struct hfg_ctx {
   int *d_task_counts = nullptr;
   int *d_queue = nullptr;  // per quartet class: the device work queue's counter
   std::vector<int> task_base;  // per quartet class, offset into d_task_active
+  hfg_stats stats{};
+  bool profiling = false;
   // a library handle of another translation unit (the MO transform's cuBLAS
   // handle), destroyed with the context
   void *handle = nullptr;
   void (*handle_destroy)(void *) = nullptr;
-  hfg_stats stats{};
-  bool profiling = false;
   bool precision_form() const { return opts.density_screening || opts.incremental || mixed_cutoff > 0; }
   double density_threshold() const {
     return opts.density_threshold > 0 ? opts.density_threshold : opts.schwarz_threshold;
@@ -461,103 +462,122 @@ static void build_group_tasks(const hfg_ctx *c, QuartetClass &q, const std::vect
 // Every unordered pair of pairs appears once: for different classes all
 // (bra, ket) combinations, for the same class the kets at positions <= the
 // bra's position in the concatenated bucket list.
+static QuartetClass build_quartet_class(const hfg_ctx *c, int ci, double threshold) {
+  const ClassEntry &ce = kClasses[ci];
+  QuartetClass q;
+  q.cls = ci;
+  q.bra_pc = pair_class_index(ce.la, ce.lb);
+  q.ket_pc = pair_class_index(ce.lc, ce.ld);
+  const PairClassList &BL = c->pclass[q.bra_pc], &KL = c->pclass[q.ket_pc];
+  const auto &bras = BL.pairs;
+  const auto &kets = KL.pairs;
+  if (bras.empty() || kets.empty()) return q;
+  const bool same = q.bra_pc == q.ket_pc;
+  std::vector<int64_t> kfun(kets.size() + 1, 0), kprim(kets.size() + 1, 0);
+  std::vector<double> kq(kets.size());
+  for (size_t k = 0; k < kets.size(); ++k) {
+    kfun[k + 1] = kfun[k] + pair_functions(c, kets[k]);
+    kprim[k + 1] = kprim[k] + c->pair_nprim[kets[k]];
+    kq[k] = c->pair_Q[kets[k]];
+  }
+  const double pf = prim_flops(ci, c->opts.eri_convention == HFG_ERI_REFERENCE);
+  const double hf = hrr_flops(ci);
+  const int ltot = ce.la + ce.lb + ce.lc + ce.ld;
+  // the longest ket contraction of each bucket segment
+  std::vector<int> segmax(KL.seg_start.size(), 0);
+  for (size_t g = 0; g + 1 < KL.seg_start.size(); ++g)
+    for (int64_t k2 = KL.seg_start[g]; k2 < KL.seg_start[g + 1]; ++k2)
+      segmax[g] = std::max(segmax[g], c->pair_nprim[kets[k2]]);
+  // fused thread-per-quartet classes: lanes per quartet so that a lane's
+  // share of a quartet's primitive quartets stays near the target (long
+  // contractions spread over 2..32 lanes, fewer kets per task); the large
+  // classes (split path: one lane per quartet; warp kernel: one warp per
+  // quartet) keep 32 kets per task
+  const bool grouped = !kSplit[ci] && !kWarp[ci];
+  // per bra and ket bucket: the end of its kets (grouped tasks)
+  std::vector<int> ends(kGroup[ci] ? bras.size() * kBuckets : 0, -1);
+  const int target = c->class_prim_target[ci] > 0 ? c->class_prim_target[ci]
+                     : c->class_prim_target[ci] < 0 ? 0 : c->prim_target;
+  for (size_t b = 0; b < bras.size(); ++b) {
+    const double qb = c->pair_Q[bras[b]];
+    if (!(qb > 0)) continue;
+    const double need = threshold / qb;
+    const int64_t bf = pair_functions(c, bras[b]);
+    const int64_t bprim = c->pair_nprim[bras[b]];
+    // kets come from the bra's own molecule only
+    const int mol = c->pair_mol.empty() ? 0 : c->pair_mol[bras[b]];
+    for (int k = 0; k < kBuckets; ++k) {
+      const int64_t s0 = KL.seg_start[mol * kBuckets + k], s1 = KL.seg_start[mol * kBuckets + k + 1];
+      // kets of the bucket with qb * qk >= threshold form a prefix
+      int64_t lo = s0, hi = s1;
+      while (lo < hi) {
+        const int64_t mid = (lo + hi) / 2;
+        if (kq[mid] >= need) lo = mid + 1;
+        else hi = mid;
+      }
+      int64_t end = lo;
+      if (same) end = std::min<int64_t>(end, (int64_t)b + 1);
+      if (end <= s0) continue;
+      if (kGroup[ci]) ends[b * kBuckets + k] = (int)end;
+      int per_task = 32;
+      if (grouped && target > 0) {
+        const double work = (double)bprim * segmax[mol * kBuckets + k];
+        int G = 1;
+        while (G < 32 && work / G > target) G <<= 1;
+        per_task = 32 / G;
+      }
+      for (int64_t st = s0; st < end; st += per_task) {
+        const int64_t e1 = std::min<int64_t>(st + per_task, end);
+        Task tk{(int)b, (int)st, (int)e1};
+        int m2 = 1;
+        while (m2 < e1 - st) m2 <<= 1;
+        if (grouped)
+          while ((32 >> tk.lg) > m2) ++tk.lg;  // 32 / 2^lg lane groups, at least the task's kets
+        q.tasks.push_back(tk);
+        int64_t mx = 0;
+        for (int64_t k2 = st; k2 < e1; ++k2) mx = std::max<int64_t>(mx, c->pair_nprim[kets[k2]]);
+        q.lane_work += (double)bprim * (double)(kprim[e1] - kprim[st]);
+        q.warp_work += 32.0 * std::ceil((double)bprim * (double)mx / (double)(1 << tk.lg));
+        if (q.cost_prefix.empty()) q.cost_prefix.push_back(0.0);
+        q.cost_prefix.push_back(q.cost_prefix.back() +
+                                (double)bprim * (double)(kprim[e1] - kprim[st]) * (pf + boys_geom_flops(ltot)) +
+                                (double)(e1 - st) * hf);
+      }
+      q.shell_quartets += end - s0;
+      if (same && end == (int64_t)b + 1) {
+        // the diagonal quartet (bra == ket) counts its unique half
+        q.function_quartets += bf * (kfun[end - 1] - kfun[s0]) + bf * (bf + 1) / 2;
+      } else {
+        q.function_quartets += bf * (kfun[end] - kfun[s0]);
+      }
+      q.prim_quartets += bprim * (kprim[end] - kprim[s0]);
+    }
+  }
+  q.flops = (double)q.prim_quartets * (pf + boys_geom_flops(ltot)) + (double)q.shell_quartets * hf;
+  if (kGroup[ci] && (int64_t)q.tasks.size() >= (int64_t)c->group_min_tasks * c->num_sms)
+    build_group_tasks(c, q, ends, segmax, kprim, target, pf + boys_geom_flops(ltot), hf);
+  return q;
+}
+
 static void build_quartet_classes(hfg_ctx *c, double threshold) {
   c->qclasses.clear();
   std::fill(std::begin(c->class_prims), std::end(c->class_prims), int64_t(0));
+  // bra order of the grouped tasks
+  for (PairClassList &L : c->pclass) {
+    if (L.gpairs.size() == L.pairs.size()) continue;
+    L.gpairs = L.pairs;
+    for (size_t x = 0; x + 1 < L.seg_start.size(); ++x)
+      std::stable_sort(L.gpairs.begin() + L.seg_start[x], L.gpairs.begin() + L.seg_start[x + 1],
+                       [&](int a, int b) { return c->pair_sa[a] < c->pair_sa[b]; });
+  }
+  // the classes' lists are independent: one thread each for large molecules
+  // ((H2O)32 / 6-31G*: 3.2 million tasks)
+  std::vector<std::future<QuartetClass>> lists;
+  const auto how = c->npairs >= 4096 ? std::launch::async : std::launch::deferred;
+  for (int ci = 0; ci < kNumClasses; ++ci)
+    lists.push_back(std::async(how, [c, ci, threshold] { return build_quartet_class(c, ci, threshold); }));
   for (int ci = 0; ci < kNumClasses; ++ci) {
-    const ClassEntry &ce = kClasses[ci];
-    QuartetClass q;
-    q.cls = ci;
-    q.bra_pc = pair_class_index(ce.la, ce.lb);
-    q.ket_pc = pair_class_index(ce.lc, ce.ld);
-    const PairClassList &BL = c->pclass[q.bra_pc], &KL = c->pclass[q.ket_pc];
-    const auto &bras = BL.pairs;
-    const auto &kets = KL.pairs;
-    if (bras.empty() || kets.empty()) continue;
-    const bool same = q.bra_pc == q.ket_pc;
-    std::vector<int64_t> kfun(kets.size() + 1, 0), kprim(kets.size() + 1, 0);
-    std::vector<double> kq(kets.size());
-    for (size_t k = 0; k < kets.size(); ++k) {
-      kfun[k + 1] = kfun[k] + pair_functions(c, kets[k]);
-      kprim[k + 1] = kprim[k] + c->pair_nprim[kets[k]];
-      kq[k] = c->pair_Q[kets[k]];
-    }
-    const double pf = prim_flops(ci, c->opts.eri_convention == HFG_ERI_REFERENCE);
-    const double hf = hrr_flops(ci);
-    const int ltot = ce.la + ce.lb + ce.lc + ce.ld;
-    // the longest ket contraction of each bucket segment
-    std::vector<int> segmax(KL.seg_start.size(), 0);
-    for (size_t g = 0; g + 1 < KL.seg_start.size(); ++g)
-      for (int64_t k2 = KL.seg_start[g]; k2 < KL.seg_start[g + 1]; ++k2)
-        segmax[g] = std::max(segmax[g], c->pair_nprim[kets[k2]]);
-    // fused thread-per-quartet classes: lanes per quartet so that a lane's
-    // share of a quartet's primitive quartets stays near the target (long
-    // contractions spread over 2..32 lanes, fewer kets per task); the large
-    // classes (split path: one lane per quartet; warp kernel: one warp per
-    // quartet) keep 32 kets per task
-    const bool grouped = !kSplit[ci] && !kWarp[ci];
-    // per bra and ket bucket: the end of its kets (grouped tasks)
-    std::vector<int> ends(kGroup[ci] ? bras.size() * kBuckets : 0, -1);
-    const int target = c->class_prim_target[ci] > 0 ? c->class_prim_target[ci]
-                       : c->class_prim_target[ci] < 0 ? 0 : c->prim_target;
-    for (size_t b = 0; b < bras.size(); ++b) {
-      const double qb = c->pair_Q[bras[b]];
-      if (!(qb > 0)) continue;
-      const double need = threshold / qb;
-      const int64_t bf = pair_functions(c, bras[b]);
-      const int64_t bprim = c->pair_nprim[bras[b]];
-      // kets come from the bra's own molecule only
-      const int mol = c->pair_mol.empty() ? 0 : c->pair_mol[bras[b]];
-      for (int k = 0; k < kBuckets; ++k) {
-        const int64_t s0 = KL.seg_start[mol * kBuckets + k], s1 = KL.seg_start[mol * kBuckets + k + 1];
-        // kets of the bucket with qb * qk >= threshold form a prefix
-        int64_t lo = s0, hi = s1;
-        while (lo < hi) {
-          const int64_t mid = (lo + hi) / 2;
-          if (kq[mid] >= need) lo = mid + 1;
-          else hi = mid;
-        }
-        int64_t end = lo;
-        if (same) end = std::min<int64_t>(end, (int64_t)b + 1);
-        if (end <= s0) continue;
-        if (kGroup[ci]) ends[b * kBuckets + k] = (int)end;
-        int per_task = 32;
-        if (grouped && target > 0) {
-          const double work = (double)bprim * segmax[mol * kBuckets + k];
-          int G = 1;
-          while (G < 32 && work / G > target) G <<= 1;
-          per_task = 32 / G;
-        }
-        for (int64_t st = s0; st < end; st += per_task) {
-          const int64_t e1 = std::min<int64_t>(st + per_task, end);
-          Task tk{(int)b, (int)st, (int)e1};
-          int m2 = 1;
-          while (m2 < e1 - st) m2 <<= 1;
-          if (grouped)
-            while ((32 >> tk.lg) > m2) ++tk.lg;  // 32 / 2^lg lane groups, at least the task's kets
-          q.tasks.push_back(tk);
-          int64_t mx = 0;
-          for (int64_t k2 = st; k2 < e1; ++k2) mx = std::max<int64_t>(mx, c->pair_nprim[kets[k2]]);
-          q.lane_work += (double)bprim * (double)(kprim[e1] - kprim[st]);
-          q.warp_work += 32.0 * std::ceil((double)bprim * (double)mx / (double)(1 << tk.lg));
-          if (q.cost_prefix.empty()) q.cost_prefix.push_back(0.0);
-          q.cost_prefix.push_back(q.cost_prefix.back() +
-                                  (double)bprim * (double)(kprim[e1] - kprim[st]) * (pf + boys_geom_flops(ltot)) +
-                                  (double)(e1 - st) * hf);
-        }
-        q.shell_quartets += end - s0;
-        if (same && end == (int64_t)b + 1) {
-          // the diagonal quartet (bra == ket) counts its unique half
-          q.function_quartets += bf * (kfun[end - 1] - kfun[s0]) + bf * (bf + 1) / 2;
-        } else {
-          q.function_quartets += bf * (kfun[end] - kfun[s0]);
-        }
-        q.prim_quartets += bprim * (kprim[end] - kprim[s0]);
-      }
-    }
-    q.flops = (double)q.prim_quartets * (pf + boys_geom_flops(ltot)) + (double)q.shell_quartets * hf;
-    if (kGroup[ci] && (int64_t)q.tasks.size() >= (int64_t)c->group_min_tasks * c->num_sms)
-      build_group_tasks(c, q, ends, segmax, kprim, target, pf + boys_geom_flops(ltot), hf);
+    QuartetClass q = lists[ci].get();
     c->class_prims[ci] = q.prim_quartets;
     if (!q.tasks.empty()) c->qclasses.push_back(std::move(q));
   }
@@ -603,7 +623,76 @@ __global__ void group_masks_kernel(const EngineView v, const int *__restrict__ b
   }
 }
 
+// Ket primitive pairs of one class's blocked list (KetField): records past a
+// pair's last one have no weight and lie at a distance from everything.
+__global__ void fill_ket_blocks(const EngineView v, const int *__restrict__ pairs, int npairs,
+                                const int *__restrict__ block_off, const int *__restrict__ block_records, int nblocks,
+                                double *__restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  for (int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nblocks; b += gridDim.x * (blockDim.x >> 5)) {
+    const int pos = 32 * b + lane, p = pos < npairs ? pairs[pos] : -1;
+    const int off = p >= 0 ? v.pair_prim_off[p] : 0, np = p >= 0 ? v.pair_nprim[p] : 0;
+    for (int i = 0; i < block_records[b]; ++i) {
+      double *o = out + (size_t)(block_off[b] + i) * kKetStride + lane;
+      PrimPair pp{};
+      if (i < np) pp = v.prim[off + i];
+      else pp.Px = 1e6;
+      o[kKetPx * 32] = pp.Px;
+      o[(kKetPx + 1) * 32] = pp.Py;
+      o[(kKetPx + 2) * 32] = pp.Pz;
+      o[kKetKf * 32] = pp.Kf;
+      o[kKetInvZeta * 32] = pp.inv_zeta;
+      o[kKetBAB * 32] = pp.bABx;
+      o[(kKetBAB + 1) * 32] = pp.bABy;
+      o[(kKetBAB + 2) * 32] = pp.bABz;
+      o[kKetZeta * 32] = pp.zeta;
+      o[kKetK * 32] = pp.K;
+    }
+  }
+}
+
+// What the grouped kernel reads of a pair class, made when the first class of
+// the context is grouped: the bra order, the list positions, the blocked list.
+static hfg_status upload_group_layout(hfg_ctx *c) {
+  hfg_status st;
+  if (c->d_pair_pos) return HFG_OK;
+  if ((st = upload(&c->d_pair_pos, c->pair_pos)) != HFG_OK) return st;
+  for (PairClassList &L : c->pclass) {
+    if (L.pairs.empty()) continue;
+    std::vector<int> segmax(L.pairs.size(), 0), off, records;
+    for (size_t x = 0; x + 1 < L.seg_start.size(); ++x) {
+      int most = 0;
+      for (int k = L.seg_start[x]; k < L.seg_start[x + 1]; ++k) most = std::max(most, c->pair_nprim[L.pairs[k]]);
+      std::fill(segmax.begin() + L.seg_start[x], segmax.begin() + L.seg_start[x + 1], most);
+    }
+    int total = 0;
+    for (size_t x = 0; x < L.pairs.size(); x += 32) {
+      // as many records as the longest contraction of a segment the block
+      // touches: a task's kets are of one segment and read alike
+      const int most = std::max(1, *std::max_element(segmax.begin() + x, segmax.begin() + std::min(x + 32, segmax.size())));
+      off.push_back(total);
+      records.push_back(most);
+      total += most;
+    }
+    int *d_records = nullptr;
+    if ((st = upload(&L.d_gpairs, L.gpairs)) != HFG_OK || (st = upload(&L.d_block_off, off)) != HFG_OK ||
+        (st = upload(&d_records, records)) != HFG_OK)
+      return st;
+    HFG_CUDA(cudaMalloc((void **)&L.d_blocks, (size_t)total * kKetStride * sizeof(double)));
+    const int nb = (int)off.size();
+    fill_ket_blocks<<<std::max(1, std::min(c->num_sms * 8, (nb + 7) / 8)), 256, 0, c->stream>>>(
+        c->view(), L.d_pairs, (int)L.pairs.size(), L.d_block_off, d_records, nb, L.d_blocks);
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    cudaFree(d_records);
+    HFG_CUDA(e);
+  }
+  return HFG_OK;
+}
+
 static hfg_status upload_classes(hfg_ctx *c) {
+  for (const auto &q : c->qclasses)
+    if (!q.gtasks.empty())
+      if (const hfg_status st = upload_group_layout(c); st != HFG_OK) return st;
   for (auto &q : c->qclasses) {
     hfg_status st = upload(&q.d_tasks, q.tasks);
     if (st != HFG_OK || (st = upload(&q.d_gtasks, q.gtasks)) != HFG_OK) return st;
@@ -1707,41 +1796,8 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
     }
     L.seg_start[seg.size()] = (int)L.pairs.size();
     for (size_t x = 0; x < L.pairs.size(); ++x) ctx->pair_pos[L.pairs[x]] = (int)x;
-    L.gpairs = L.pairs;
-    for (size_t x = 0; x < seg.size(); ++x)
-      std::stable_sort(L.gpairs.begin() + L.seg_start[x], L.gpairs.begin() + L.seg_start[x + 1],
-                       [&](int a, int b) { return ctx->pair_sa[a] < ctx->pair_sa[b]; });
-    std::vector<int> segmax_of(L.pairs.size(), 0);
-    for (size_t x = 0; x < seg.size(); ++x) {
-      int most = 0;
-      for (int p : seg[x]) most = std::max(most, pn[p]);
-      std::fill(segmax_of.begin() + L.seg_start[x], segmax_of.begin() + L.seg_start[x + 1], most);
-    }
-    std::vector<int> boff;
-    std::vector<double> blocks;
-    for (size_t x = 0; x < L.pairs.size(); x += 32) {
-      const size_t rec = blocks.size() / kKetStride, end = std::min(x + 32, L.pairs.size());
-      boff.push_back((int)rec);
-      // as many records as the longest contraction of a segment the block
-      // touches: a task's kets are of one segment and read alike
-      int most = 1;
-      for (size_t y = x; y < end; ++y) most = std::max(most, segmax_of[y]);
-      blocks.resize((rec + most) * kKetStride, 0.0);
-      // records past a pair's last one: no weight, at a distance from everything
-      for (size_t r = rec; r < rec + most; ++r)
-        for (int k = 0; k < 32; ++k) blocks[r * kKetStride + kKetPx * 32 + k] = 1e6;
-      for (size_t y = x; y < end; ++y)
-        for (int i = 0; i < pn[L.pairs[y]]; ++i) {
-          const PrimPair &pp = prim[poff[L.pairs[y]] + i];
-          const double f[kKetFields] = {pp.Px, pp.Py, pp.Pz, pp.Kf, pp.inv_zeta, pp.bABx, pp.bABy, pp.bABz, pp.zeta, pp.K};
-          for (int k = 0; k < kKetFields; ++k) blocks[(rec + i) * kKetStride + k * 32 + (y - x)] = f[k];
-        }
-    }
-    if ((st = upload(&L.d_pairs, L.pairs)) != HFG_OK || (st = upload(&L.d_gpairs, L.gpairs)) != HFG_OK ||
-        (st = upload(&L.d_blocks, blocks)) != HFG_OK || (st = upload(&L.d_block_off, boff)) != HFG_OK)
-      return st;
+    if ((st = upload(&L.d_pairs, L.pairs)) != HFG_OK) return st;
   }
-  if ((st = upload(&ctx->d_pair_pos, ctx->pair_pos)) != HFG_OK) return st;
   build_quartet_classes(ctx.get(), ctx->opts.schwarz_threshold);
   if ((st = upload_classes(ctx.get())) != HFG_OK) return st;
   if (ctx->batch) {
