@@ -162,6 +162,15 @@ def _oracle():
     return O
 
 
+def _reference_missing():
+    """Why the reference cannot be timed here (None: it can)."""
+    try:
+        _oracle()
+    except RuntimeError as e:
+        return str(e)
+    return None
+
+
 def reference_rate(sample_per_thread: int, threads: int, waters: int) -> dict:
     """The reference's own CPU ERI path (IntegralsRepository::getElectronElectron,
     one repository per thread) on quartets drawn uniformly from every 8-fold
@@ -363,6 +372,10 @@ def batching(count: int, check: int = 8):
 
 def run_reference_arm(args, rank, world):
     if rank != 0:
+        return 0
+    missing = _reference_missing()
+    if missing:
+        print(json.dumps({"impl": "reference", "unavailable": missing}), flush=True)
         return 0
     threads = os.cpu_count() or 1
     per_step, last = [], None
@@ -663,14 +676,17 @@ def main():
         line["scf"] = scf_comparison(args.scf_waters)
     if rank == 0 and world == 1 and not args.no_reference_scf:
         from hartreefock_b200 import molecules
-        line["scf_vs_reference"] = reference_scf([
+        missing = _reference_missing()
+        line["scf_vs_reference"] = {"unavailable": missing} if missing else reference_scf([
             ("H2O (README geometry)", molecules.H2O_README, "sto-3g", 0.5, 0.0),
             ("(H2O)_2 seed 0", molecules.water_cluster(2, seed=0), "6-31g*", 0.75, 0.75)])
     if rank == 0 and world == 1 and args.serve_jobs > 0:
         line["serving"] = serving(args.serve_jobs)
     if rank == 0 and world == 1 and args.batch_mols > 0:
         line["batching"] = batching(args.batch_mols)
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and _reference_missing():
+        line["cpu_baseline"] = {"unavailable": _reference_missing()}
+    elif rank == 0 and world == 1 and not args.no_cpu_baseline:
         cb = reference_rate(args.ref_sample, 1, WATERS)
         line["cpu_baseline"] = {"value": cb["value"], "unit": "quartets/s", "cores": 1, "kind": "reference",
                                 "sample": f"{cb['sampled_quartets']} quartets drawn uniformly from all "
