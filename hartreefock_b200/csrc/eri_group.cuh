@@ -25,8 +25,9 @@
 // Per (H2O)32 / 6-31G* build, classes one after another, before and now:
 // (ps|ss) 4.36 -> 3.05 ms, (ss|ss) 2.70 -> 1.85, (ds|ps) 2.17 -> 1.83, (ds|ss)
 // 1.97 -> 1.42, (ps|ps) 1.77 -> 1.57, (dp|ss) 1.06 -> 0.79.  (ps|ss) now issues on
-// 45% of the cycles (26% before) and runs the FP64 pipe at 27%; it waits on L1
-// misses (3.1 of 8.2 warps per issue) and fixed latencies (2.3).  Switched off in
+// 47% of the cycles (26% before), with the FP64 pipe at 31% and the L1 data pipe
+// at 62%; it waits on L1 misses (2.8 of 8.0 warps per issue) and fixed latencies
+// (2.2).  Switched off in
 // turn there, the near loop takes 1.4 ms, the far loop 1.3 ms and the digestion
 // 0.35 ms.
 #pragma once

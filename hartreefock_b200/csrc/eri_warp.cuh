@@ -13,8 +13,8 @@
 //   2. the contracted [e0|f0] block goes to shared memory and the lanes
 //      expand it into the normalised (ab|cd) block there, element by element
 //      with the horizontal recursions as tables (HrrTable): every lane runs the
-//      same code.  (A row (a b) per lane ran the generated row code, a switch
-//      over the rows, one lane at a time.);
+//      same code (a row (a b) per lane ran the generated row code, a switch
+//      over the rows, one lane at a time);
 //   3. the lanes digest the block: every element of J_ab, J_cd, K_ac, K_ad,
 //      K_bc, K_bd is one lane's dot product over the block, then one atomic
 //      (or the packed-table store).  The density entries are read side by side

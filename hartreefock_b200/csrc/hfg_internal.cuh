@@ -114,9 +114,10 @@ __host__ __device__ constexpr int group_warps(int la, int lb, int lc, int ld) {
 // 156 against 52, 58, 69 (4,541 in (H2O)4); (dp|pp) 78, 109 against 94, 104 (3,994 in
 // (H2O)4); (dp|ds) is level at 470.  (dd|dd) is faster here at every size (0.24
 // against 0.82 ms at (H2O)16, before its recursions became tables).  (dp|dp) would
-// gain too (56 against 157 at (H2O)2), but its transfer in this kernel's
-// association is 3.1e-12 off on two cancelling elements of O2 / 6-31G* (1.3e-12 on
-// the split path), so it stays where it was.
+// gain too (56 against 157 at (H2O)2), but this kernel is 3.1e-12 off the
+// reference on two cancelling elements of O2 / 6-31G* (1.3e-12 on the split path;
+// adding the transfer terms one by one as the per-thread code does changes
+// nothing), so it stays where it was.
 __host__ __device__ constexpr long long warp_prim_limit(int la, int lb, int lc, int ld) {
   const int ket = 10 * lc + ld;
   if (la == 2 && lb == 2)
