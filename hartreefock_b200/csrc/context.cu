@@ -573,7 +573,8 @@ static void build_quartet_classes(hfg_ctx *c, double threshold) {
   // the classes' lists are independent: one thread each for large molecules
   // ((H2O)32 / 6-31G*: 3.2 million tasks)
   std::vector<std::future<QuartetClass>> lists;
-  const auto how = c->npairs >= 4096 ? std::launch::async : std::launch::deferred;
+  // (or on this one, where no thread is to be had)
+  const auto how = c->npairs >= 4096 ? std::launch::async | std::launch::deferred : std::launch::deferred;
   for (int ci = 0; ci < kNumClasses; ++ci)
     lists.push_back(std::async(how, [c, ci, threshold] { return build_quartet_class(c, ci, threshold); }));
   for (int ci = 0; ci < kNumClasses; ++ci) {
