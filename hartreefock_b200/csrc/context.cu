@@ -394,6 +394,10 @@ static inline int64_t pair_functions(const hfg_ctx *c, int p) {
   return c->pair_sa[p] == c->pair_sb[p] ? (int64_t)na * (na + 1) / 2 : (int64_t)na * nb;
 }
 
+// SMs the grouped lists are made for.  A constant, so that every rank of a
+// sharded build makes the same lists.
+constexpr int kGroupSms = 148;
+
 // Grouped tasks of one class (eri_group.cuh): every run of bras with one first
 // shell (same molecule and primitive bucket) against every chunk of kets of a
 // bucket that one of them reaches.  `ends`: per bra position and ket bucket the
@@ -404,7 +408,7 @@ static void build_group_tasks(const hfg_ctx *c, QuartetClass &q, const std::vect
   const PairClassList &BL = c->pclass[q.bra_pc], &KL = c->pclass[q.ket_pc];
   const auto &bras = BL.gpairs;
   // bras per task: as many as leave several tasks for every warp of the GPU
-  const int most = (int)std::max<int64_t>(1, std::min<int64_t>(kGroupMaxBras, (int64_t)q.tasks.size() / (c->num_sms * 96)));
+  const int most = (int)std::max<int64_t>(1, std::min<int64_t>(kGroupMaxBras, (int64_t)q.tasks.size() / (kGroupSms * 96)));
   q.gtasks.clear();
   q.gcost_prefix.assign(1, 0.0);
   q.ngmasks = 0;
@@ -554,7 +558,7 @@ static QuartetClass build_quartet_class(const hfg_ctx *c, int ci, double thresho
     }
   }
   q.flops = (double)q.prim_quartets * (pf + boys_geom_flops(ltot)) + (double)q.shell_quartets * hf;
-  if (kGroup[ci] && (int64_t)q.tasks.size() >= (int64_t)c->group_min_tasks * c->num_sms)
+  if (kGroup[ci] && (int64_t)q.tasks.size() >= (int64_t)c->group_min_tasks * kGroupSms)
     build_group_tasks(c, q, ends, segmax, kprim, target, pf + boys_geom_flops(ltot), hf);
   return q;
 }
@@ -788,10 +792,15 @@ static double launch_share(const QuartetClass &q, const ClassLaunch &cl) {
   return (prefix[cl.task_offset + cl.ntasks] - prefix[cl.task_offset]) / prefix.back();
 }
 
-// plain FP64 J/K builds of the class run the grouped kernel (kGroupMinTasks)
+// Plain FP64 J/K builds of the class run the grouped kernel (kGroupMinTasks:
+// the line, twice that on concurrent streams).  A shard's line is the higher
+// one whatever the context's streams: a shard is a range of the list that its
+// kernel walks, so every rank must take the same list, and a rank has a part
+// of the tasks only.
 static bool uses_group(const hfg_ctx *c, const QuartetClass &q) {
   if (q.gtasks.empty()) return false;
-  return !c->use_streams || c->profiling || (int64_t)q.tasks.size() >= 2 * (int64_t)c->group_min_tasks * c->num_sms;
+  const int64_t line = (int64_t)c->group_min_tasks * kGroupSms;
+  return (int64_t)q.tasks.size() >= (c->use_streams || c->shard_count > 1 ? 2 * line : line);
 }
 
 __global__ void finalize_rhf(const double *J, const double *K, double *G, int n) {

@@ -17,7 +17,8 @@ class ShardedFock:
     and fock_uhf_tensor(Pa, Pb, Ga, Gb) (hartreefock_b200.engine.Engine).
     Shards are ranges of each class's task list, so every rank's engine must
     hold the same task lists: the same molecule, options and lane-group
-    targets (no per-rank Engine.autotune_tasks / set_prim_target choices)."""
+    targets (no per-rank Engine.autotune_tasks / set_prim_target choices).
+    Class streams, graphs and per-class timing may differ between ranks."""
 
     def __init__(self, engine, group=None):
         import torch.distributed as dist

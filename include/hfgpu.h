@@ -172,7 +172,10 @@ hfg_status hfg_set_incremental(hfg_ctx *ctx, int32_t on);
  * class's per-primitive flops, plus its per-quartet horizontal recursions),
  * and return that shard's partial G.  The partial G of the `count` shards
  * sum to the full G (G is linear in the J/K sums); the caller reduces them,
- * e.g. with one NCCL all-reduce (hartreefock_b200/shards.py).  Incremental
+ * e.g. with one NCCL all-reduce (hartreefock_b200/shards.py).  The ranges are
+ * cut from the class's task list: the same on every rank with the same
+ * molecule, hfg_opts and lane-group targets, whatever its class streams,
+ * graphs, per-class timing, grids and class paths.  Incremental
  * builds keep a per-shard history.  Stored builds (hfg_eri_packed) and
  * hfg_fock_rhf_noalloc are not sharded.  Default (0, 1). */
 hfg_status hfg_set_shard(hfg_ctx *ctx, int32_t rank, int32_t count);
