@@ -39,9 +39,11 @@ const std::vector<double> &boys_table_for_external() { return boys_table_host();
 #define HFG_CUDA(call)                                                                        \
   do {                                                                                        \
     cudaError_t err__ = (call);                                                               \
-    if (err__ != cudaSuccess)                                                                 \
+    if (err__ != cudaSuccess) {                                                               \
+      cudaGetLastError(); /* reported here: not again by the next launch's check */            \
       return fail(err__ == cudaErrorMemoryAllocation ? HFG_OOM_BUDGET : HFG_DEVICE_ERROR,      \
                   std::string(#call) + ": " + cudaGetErrorString(err__));                     \
+    }                                                                                         \
   } while (0)
 
 // ---------------------------------------------------------------------------
@@ -146,6 +148,14 @@ static hfg_status upload(T **dst, const std::vector<T> &src) {
   return HFG_OK;
 }
 
+// Device buffers freed at the end of a scope.
+struct Scoped {
+  std::vector<void *> ptrs;
+  ~Scoped() {
+    for (void *p : ptrs) cudaFree(p);
+  }
+};
+
 }  // namespace hfg
 
 using namespace hfg;
@@ -161,6 +171,8 @@ struct hfg_ctx {
   std::vector<double> pair_Q;
   PairClassList pclass[kNumPairClasses];
   std::vector<QuartetClass> qclasses;
+  bool lists_ready = false;   // qclasses and their device lists are complete
+  bool group_layout = false;  // so is what upload_group_layout makes
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // class kernels of one build are independent (J/K by atomics): they run on
@@ -656,11 +668,22 @@ __global__ void fill_ket_blocks(const EngineView v, const int *__restrict__ pair
   }
 }
 
-// What the grouped kernel reads of a pair class, made when the first class of
-// the context is grouped: the bra order, the list positions, the blocked list.
-static hfg_status upload_group_layout(hfg_ctx *c) {
+static void free_group_layout(hfg_ctx *c) {
+  cudaFree(c->d_pair_pos);
+  c->d_pair_pos = nullptr;
+  for (PairClassList &L : c->pclass) {
+    cudaFree(L.d_gpairs);
+    cudaFree(L.d_blocks);
+    cudaFree(L.d_block_off);
+    L.d_gpairs = nullptr;
+    L.d_blocks = nullptr;
+    L.d_block_off = nullptr;
+  }
+  c->group_layout = false;
+}
+
+static hfg_status make_group_layout(hfg_ctx *c) {
   hfg_status st;
-  if (c->d_pair_pos) return HFG_OK;
   if ((st = upload(&c->d_pair_pos, c->pair_pos)) != HFG_OK) return st;
   for (PairClassList &L : c->pclass) {
     if (L.pairs.empty()) continue;
@@ -680,18 +703,37 @@ static hfg_status upload_group_layout(hfg_ctx *c) {
       total += most;
     }
     int *d_records = nullptr;
-    if ((st = upload(&L.d_gpairs, L.gpairs)) != HFG_OK || (st = upload(&L.d_block_off, off)) != HFG_OK ||
-        (st = upload(&d_records, records)) != HFG_OK)
+    Scoped tmp;
+    st = upload(&d_records, records);
+    tmp.ptrs.push_back(d_records);
+    if (st != HFG_OK || (st = upload(&L.d_gpairs, L.gpairs)) != HFG_OK || (st = upload(&L.d_block_off, off)) != HFG_OK)
       return st;
     HFG_CUDA(cudaMalloc((void **)&L.d_blocks, (size_t)total * kKetStride * sizeof(double)));
     const int nb = (int)off.size();
     fill_ket_blocks<<<std::max(1, std::min(c->num_sms * 8, (nb + 7) / 8)), 256, 0, c->stream>>>(
         c->view(), L.d_pairs, (int)L.pairs.size(), L.d_block_off, d_records, nb, L.d_blocks);
-    const cudaError_t e = cudaStreamSynchronize(c->stream);
-    cudaFree(d_records);
-    HFG_CUDA(e);
+    HFG_CUDA(cudaGetLastError());
+    HFG_CUDA(cudaStreamSynchronize(c->stream));
   }
   return HFG_OK;
+}
+
+// What the grouped kernel reads of a pair class, made when the first class of
+// the context is grouped: the bra order, the list positions, the blocked list.
+// All of it or, on a failure, nothing.
+static hfg_status upload_group_layout(hfg_ctx *c) {
+  if (c->group_layout) return HFG_OK;
+  const hfg_status st = make_group_layout(c);
+  if (st != HFG_OK) free_group_layout(c);
+  c->group_layout = st == HFG_OK;
+  return st;
+}
+
+// A build needs the lists: an error where a rebuild of them failed.
+static hfg_status need_lists(const hfg_ctx *c) {
+  return c->lists_ready ? HFG_OK
+                        : fail(HFG_DEVICE_ERROR, "the context has no task lists: rebuilding them failed "
+                                                 "(hfg_set_prim_target tries again)");
 }
 
 static hfg_status upload_classes(hfg_ctx *c) {
@@ -711,6 +753,7 @@ static hfg_status upload_classes(hfg_ctx *c) {
     HFG_CUDA(cudaGetLastError());
   }
   HFG_CUDA(cudaStreamSynchronize(c->stream));
+  c->lists_ready = true;
   return HFG_OK;
 }
 
@@ -1179,6 +1222,7 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
 // change of buffers, stream or settings starts over.
 static hfg_status direct_build(hfg_ctx *c, bool uhf, const double *dPa, const double *dPb, double *dGa, double *dGb,
                                cudaStream_t s) {
+  if (const hfg_status st = need_lists(c); st != HFG_OK) return st;
   const bool graphable = c->use_graphs && !c->batch && !c->precision_form() && !c->profiling && s != nullptr &&
                          s != cudaStreamLegacy && s != cudaStreamPerThread;
   if (!graphable) return direct_build_body(c, uhf, dPa, dPb, dGa, dGb, s, false);
@@ -1316,6 +1360,7 @@ static hfg_status batch_build(hfg_ctx *c, bool uhf, const double *dPa, const dou
                               const unsigned char *active, cudaStream_t s) {
   const size_t tot = (size_t)c->batch_elems;
   hfg_status st;
+  if ((st = need_lists(c)) != HFG_OK) return st;
   if ((st = ensure(&c->d_J, tot)) != HFG_OK || (st = ensure(&c->d_Ka, tot)) != HFG_OK) return st;
   if (uhf && ((st = ensure(&c->d_Kb, tot)) != HFG_OK || (st = ensure(&c->d_Pt, tot)) != HFG_OK)) return st;
   const std::vector<unsigned char> all(c->nmol, 1);
@@ -1426,6 +1471,7 @@ static hfg_status batch_build_async(hfg_ctx *c, bool uhf, const double *dPa, con
   const size_t tot = (size_t)c->batch_elems;
   const size_t nq = c->qclasses.size();
   hfg_status st;
+  if ((st = need_lists(c)) != HFG_OK) return st;
   if ((st = ensure(&c->d_J, tot)) != HFG_OK || (st = ensure(&c->d_Ka, tot)) != HFG_OK) return st;
   if (uhf && ((st = ensure(&c->d_Kb, tot)) != HFG_OK || (st = ensure(&c->d_Pt, tot)) != HFG_OK)) return st;
   if ((st = ensure_task_scratch(c)) != HFG_OK) return st;
@@ -1510,6 +1556,7 @@ static hfg_status finish_timing(hfg_ctx *c) {
 
 static hfg_status stored_build(hfg_ctx *c, double *d_out, int64_t count, cudaStream_t s) {
   if (c->batch) return fail(HFG_INVALID_ARG, "batched context: no stored table");
+  if (const hfg_status st = need_lists(c); st != HFG_OK) return st;
   HFG_CUDA(cudaMemsetAsync(d_out, 0, (size_t)count * sizeof(double), s));
   HFG_CUDA(cudaEventRecord(c->ev0, s));
   const bool ref = c->opts.eri_convention == HFG_ERI_REFERENCE;
@@ -1770,18 +1817,18 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
   std::vector<std::vector<int>> by_class(kNumPairClasses);
   for (int p = 0; p < np; ++p) by_class[ctx->pair_cls[p]].push_back(p);
   const EngineView v0 = ctx->view();
-  std::vector<int *> tmp_lists;
+  Scoped tmp_lists;
   for (int pc = 0; pc < kNumPairClasses; ++pc) {
     if (by_class[pc].empty()) continue;
     int *d_list = nullptr;
-    if ((st = upload(&d_list, by_class[pc])) != HFG_OK) return st;
-    tmp_lists.push_back(d_list);
+    st = upload(&d_list, by_class[pc]);
+    tmp_lists.ptrs.push_back(d_list);
+    if (st != HFG_OK) return st;
     launch_schwarz(kPairClasses[pc][0], kPairClasses[pc][1], v0, d_list, (int)by_class[pc].size(), ctx->d_pair_Q,
                    ctx->stream);
   }
   HFG_CUDA(cudaGetLastError());
   HFG_CUDA(cudaStreamSynchronize(ctx->stream));
-  for (int *l : tmp_lists) cudaFree(l);
   ctx->pair_Q.resize(np);
   HFG_CUDA(cudaMemcpy(ctx->pair_Q.data(), ctx->d_pair_Q, (size_t)np * sizeof(double), cudaMemcpyDeviceToHost));
 
@@ -2152,6 +2199,7 @@ hfg_status hfg_autotune(hfg_ctx *c, const double *dP, int32_t *chosen, int32_t c
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c->stream;
   const size_t tot = c->batch ? (size_t)c->batch_elems : (size_t)c->nbf * c->nbf;
   hfg_status st;
+  if ((st = need_lists(c)) != HFG_OK) return st;
   if ((st = ensure(&c->d_J, tot)) != HFG_OK || (st = ensure(&c->d_Ka, tot)) != HFG_OK) return st;
   if (c->batch) {
     const std::vector<unsigned char> all(c->nmol, 1);
@@ -2259,8 +2307,7 @@ namespace hfg {
 // Rebuilds every class's task list (after a change of the lane-group
 // target): host lists, device copies, and the batched builds' compaction
 // buffers, which are sized from the lists.
-static hfg_status rebuild_tasks(hfg_ctx *c) {
-  HFG_CUDA(cudaDeviceSynchronize());  // queued builds may still read the old lists
+static void free_classes(hfg_ctx *c) {
   for (auto &q : c->qclasses) {
     cudaFree(q.d_tasks);
     cudaFree(q.d_gtasks);
@@ -2268,14 +2315,7 @@ static hfg_status rebuild_tasks(hfg_ctx *c) {
     if (q.ev_a) cudaEventDestroy(q.ev_a);
     if (q.ev_b) cudaEventDestroy(q.ev_b);
   }
-  build_quartet_classes(c, c->opts.schwarz_threshold);
-  hfg_status st = upload_classes(c);
-  if (st != HFG_OK) return st;
-  if (c->profiling)
-    for (auto &q : c->qclasses) {
-      HFG_CUDA(cudaEventCreate(&q.ev_a));
-      HFG_CUDA(cudaEventCreate(&q.ev_b));
-    }
+  c->qclasses.clear();
   cudaFree(c->d_task_active);
   cudaFree(c->d_task_counts);
   cudaFree(c->d_queue);
@@ -2283,7 +2323,26 @@ static hfg_status rebuild_tasks(hfg_ctx *c) {
   c->d_task_counts = nullptr;
   c->d_queue = nullptr;
   c->task_base.clear();
-  ++c->config_version;
+  c->lists_ready = false;
+  ++c->config_version;  // a captured graph holds the freed lists
+}
+
+// (a failure leaves the context without lists, see need_lists, and the next
+// rebuild starts from there)
+static hfg_status rebuild_tasks(hfg_ctx *c) {
+  HFG_CUDA(cudaDeviceSynchronize());  // queued builds may still read the old lists
+  free_classes(c);
+  build_quartet_classes(c, c->opts.schwarz_threshold);
+  const hfg_status st = upload_classes(c);
+  if (st != HFG_OK) {
+    free_classes(c);
+    return st;
+  }
+  if (c->profiling)
+    for (auto &q : c->qclasses) {
+      HFG_CUDA(cudaEventCreate(&q.ev_a));
+      HFG_CUDA(cudaEventCreate(&q.ev_b));
+    }
   return HFG_OK;
 }
 }  // namespace hfg
@@ -2384,6 +2443,7 @@ hfg_status hfg_autotune_paths(hfg_ctx *c, const double *dP, int32_t *chosen, int
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c->stream;
   const size_t nn = (size_t)c->nbf * c->nbf;
   hfg_status st;
+  if ((st = need_lists(c)) != HFG_OK) return st;
   if ((st = ensure(&c->d_J, nn)) != HFG_OK || (st = ensure(&c->d_Ka, nn)) != HFG_OK) return st;
   const bool ref = c->opts.eri_convention == HFG_ERI_REFERENCE;
   int written = 0;
@@ -2521,6 +2581,7 @@ extern "C" hfg_status hfg_fock_rhf_noalloc(hfg_ctx *c, const double *dP, double 
     return fail(HFG_INVALID_ARG, "hfg_fock_rhf_noalloc: " + std::to_string(c->nbf) +
                                      " basis functions exceed its fixed scratch of " +
                                      std::to_string(kNoAllocMaxNbf) + " (use hfg_fock_rhf_device)");
+  if (const hfg_status no = need_lists(c); no != HFG_OK) return no;
   HFG_CUDA(cudaSetDevice(c->device));
   double *scratch = nullptr;
   hfg_status st = noalloc_scratch(c->device, &scratch);

@@ -1,0 +1,122 @@
+"""The library's host code over a stand-in for the CUDA runtime
+(tests/fake_cuda.cpp): allocations that fail while the task lists are rebuilt.
+No kernel runs; every pointer that a launch, copy or graph replay would read is
+checked against the live allocations.  Each case runs in a process of its own,
+over the objects of the last build."""
+import ctypes
+import glob
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+if __name__ == "__main__":
+    sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+from hartreefock_b200 import engine as E
+from hartreefock_b200 import molecules
+from hartreefock_b200.build import BUILD
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CUDA = "/usr/local/cuda"
+
+
+@pytest.fixture(scope="module")
+def fake_library(tmp_path_factory):
+    objects = sorted(glob.glob(os.path.join(BUILD, "*.o")))
+    if not objects:
+        pytest.skip("no objects: python -m hartreefock_b200.build")
+    d = tmp_path_factory.mktemp("fake_cuda")
+    lib = str(d / "libhfgpu_fake.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-w", "-fPIC", f"-I{CUDA}/include", "-c",
+                    os.path.join(HERE, "fake_cuda.cpp"), "-o", str(d / "fake.o")], check=True)
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", lib, str(d / "fake.o"), *objects, f"-L{CUDA}/lib64",
+                    "-lcublas", "-lcusolver"], check=True)
+    yield lib
+    os.remove(lib)
+
+
+def _load(path):
+    L = E.library(path)
+    L.fake_complaints.restype = L.fake_log.restype = ctypes.c_char_p
+    L.fake_live_bytes.restype = L.fake_peak_bytes.restype = ctypes.c_longlong
+    return L
+
+
+def _sound(L):
+    text = L.fake_complaints().decode()
+    assert not text, text
+
+
+# --- cases, each in a child process -------------------------------------------------
+def rebuild_survives_failed_allocations(L):
+    os.environ["HFG_GROUP_MIN_TASKS"] = "0"
+    Z, xyz = molecules.water_cluster(2, seed=1)
+    P = np.eye(26)
+    for graphs in (False, True):
+        for n in range(1, 200):
+            eng = E.Engine(Z, xyz, "6-31g")
+            eng.set_graphs(graphs)
+            for _ in range(3):  # the third replays a graph
+                eng.fock_rhf(P)
+            L.fake_fail_allocation(n)
+            try:
+                eng.set_prim_target(8)
+                failed = False
+            except E.HfgError as e:
+                failed = True
+                assert e.status == 3, e
+            L.fake_fail_allocation(0)
+            if failed:
+                # nothing to build from: an error, not a launch and not a G
+                before = L.fake_launches()
+                for call in (lambda: eng.fock_rhf(P), lambda: eng.fock_uhf(P, P), eng.eri_packed):
+                    with pytest.raises(E.HfgError):
+                        call()
+                assert L.fake_launches() == before
+                eng.set_prim_target(8)  # with memory again, all is well
+            for _ in range(3):
+                eng.fock_rhf(P)
+            eng.fock_uhf(P, P)
+            _sound(L)
+            live = L.fake_live_bytes()
+            eng.close()
+            assert L.fake_live_bytes() < live
+            if not failed:
+                break
+        assert not failed and n > 10
+
+
+def context_gives_everything_back(L):
+    os.environ["HFG_GROUP_MIN_TASKS"] = "0"
+    Z, xyz = molecules.water_cluster(2, seed=1)
+    for n in range(0, 400):
+        start = L.fake_live_bytes()
+        L.fake_fail_allocation(n)
+        try:
+            eng = E.Engine(Z, xyz, "6-31g")
+        except E.HfgError:
+            eng = None
+        L.fake_fail_allocation(0)
+        if eng:
+            eng.close()
+        assert L.fake_live_bytes() == start, n
+        _sound(L)
+        if n and eng:
+            break
+    assert n > 10
+
+
+CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back)]
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_host_code(fake_library, case):
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), fake_library, case], capture_output=True, text=True,
+                       timeout=600)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+if __name__ == "__main__":
+    globals()[sys.argv[2]](_load(sys.argv[1]))
