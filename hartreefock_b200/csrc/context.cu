@@ -34,6 +34,7 @@ hfg_status fail_external(hfg_status st, const std::string &msg) { return fail(st
 static const std::vector<double> &boys_table_host();
 void *ctx_handle(hfg_ctx *c);
 void ctx_keep_handle(hfg_ctx *c, void *h, void (*destroy)(void *));
+hfg_status ctx_select(const hfg_ctx *c);
 const std::vector<double> &boys_table_for_external() { return boys_table_host(); }
 
 #define HFG_CUDA(call)                                                                        \
@@ -347,6 +348,10 @@ struct hfg_ctx {
 
 namespace hfg {
 void *ctx_handle(hfg_ctx *c) { return c->handle; }
+hfg_status ctx_select(const hfg_ctx *c) {
+  HFG_CUDA(cudaSetDevice(c->device));
+  return HFG_OK;
+}
 void ctx_keep_handle(hfg_ctx *c, void *h, void (*destroy)(void *)) {
   c->handle = h;
   c->handle_destroy = destroy;
@@ -2200,6 +2205,7 @@ hfg_status hfg_autotune(hfg_ctx *c, const double *dP, int32_t *chosen, int32_t c
   const size_t tot = c->batch ? (size_t)c->batch_elems : (size_t)c->nbf * c->nbf;
   hfg_status st;
   if ((st = need_lists(c)) != HFG_OK) return st;
+  HFG_CUDA(cudaSetDevice(c->device));
   if ((st = ensure(&c->d_J, tot)) != HFG_OK || (st = ensure(&c->d_Ka, tot)) != HFG_OK) return st;
   if (c->batch) {
     const std::vector<unsigned char> all(c->nmol, 1);
@@ -2330,6 +2336,7 @@ static void free_classes(hfg_ctx *c) {
 // (a failure leaves the context without lists, see need_lists, and the next
 // rebuild starts from there)
 static hfg_status rebuild_tasks(hfg_ctx *c) {
+  HFG_CUDA(cudaSetDevice(c->device));
   HFG_CUDA(cudaDeviceSynchronize());  // queued builds may still read the old lists
   free_classes(c);
   build_quartet_classes(c, c->opts.schwarz_threshold);
@@ -2369,6 +2376,7 @@ hfg_status hfg_autotune_tasks(hfg_ctx *c, const double *dP, int32_t *chosen, int
   cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : c->stream;
   const size_t nn = (size_t)c->nbf * c->nbf;
   hfg_status st;
+  HFG_CUDA(cudaSetDevice(c->device));
   if ((st = ensure(&c->d_J, nn)) != HFG_OK || (st = ensure(&c->d_Ka, nn)) != HFG_OK) return st;
   const bool ref = c->opts.eri_convention == HFG_ERI_REFERENCE;
   const int cand[] = {0, 48, 96, 192, 384};
@@ -2444,6 +2452,7 @@ hfg_status hfg_autotune_paths(hfg_ctx *c, const double *dP, int32_t *chosen, int
   const size_t nn = (size_t)c->nbf * c->nbf;
   hfg_status st;
   if ((st = need_lists(c)) != HFG_OK) return st;
+  HFG_CUDA(cudaSetDevice(c->device));
   if ((st = ensure(&c->d_J, nn)) != HFG_OK || (st = ensure(&c->d_Ka, nn)) != HFG_OK) return st;
   const bool ref = c->opts.eri_convention == HFG_ERI_REFERENCE;
   int written = 0;

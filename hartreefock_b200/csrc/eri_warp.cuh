@@ -26,6 +26,8 @@
 // Nothing is written to global memory but the outputs: no scratch.
 #pragma once
 
+#include <atomic>
+
 #include "eri_kernels.cuh"
 #include "eri_split_gen.cuh"
 #include "eri_warp_gen.cuh"
@@ -83,6 +85,7 @@ __device__ __forceinline__ void boys_global(double *F, double T, double scale, c
 // Shared-memory footprint of one warp, in bytes: the program's slots and the
 // contracted block(s) in R, the normalised (ab|cd) block in FP64 with rows
 // padded to an odd length (conflict-free column reads).
+constexpr int kMaxDevices = 64;  // devices whose launch shape is remembered
 constexpr int kHrrMonomials = 11;  // monomials of HrrTable's terms
 
 template <int LA, int LB, int LC, int LD, bool REF>
@@ -424,21 +427,23 @@ template <int LA, int LB, int LC, int LD, int MODE, bool REF, int SCR>
 void launch_warp(const EngineView &v, const ClassLaunch &cl, int grid, cudaStream_t s) {
   using S = WarpShape<LA, LB, LC, LD, REF>;
   auto kern = eri_warp_kernel<LA, LB, LC, LD, MODE, REF, SCR>;
-  static int resident = 0;  // blocks per SM, set once per instantiation
-  static int num_sms = 0;
-  if (resident == 0) {
+  // blocks at once on each device, set by its first launch there
+  static std::atomic<int> at_once[kMaxDevices] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  int most = dev < kMaxDevices ? at_once[dev].load() : 0;
+  if (most == 0) {
     if (S::kBytes * S::kWarps > 48 * 1024)
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kBytes * S::kWarps);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
-    int r = 0;
+    int sms = 0, r = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, kern, 32 * S::kWarps, S::kBytes * S::kWarps);
-    resident = r > 0 ? r : 1;
+    most = sms * (r > 0 ? r : 1);
+    if (dev < kMaxDevices) at_once[dev].store(most);
   }
   const long long units = (long long)cl.ntasks * 32;
   const long long need = (units + S::kWarps - 1) / S::kWarps;
-  long long g = (long long)num_sms * resident;
+  long long g = most;
   if (grid > 0) g = std::min<long long>(g, grid);
   g = std::max<long long>(1, std::min(g, need));
   kern<<<(int)g, 32 * S::kWarps, S::kBytes * S::kWarps, s>>>(v, cl);

@@ -34,6 +34,8 @@ hfg_status fail_external(hfg_status st, const std::string &msg);
 // nullptr; keep() stores it with the function that destroys it
 void *ctx_handle(hfg_ctx *c);
 void ctx_keep_handle(hfg_ctx *c, void *h, void (*destroy)(void *));
+// makes the context's device the current one: before anything is allocated or created
+hfg_status ctx_select(const hfg_ctx *c);
 }
 
 namespace {
@@ -258,6 +260,7 @@ hfg_status transform(hfg_ctx *ctx, const double *dC, int i0, int ni, int a0, int
 extern "C" hfg_status hfg_mo_eri_ovov(hfg_ctx *ctx, const double *dC, int32_t i0, int32_t ni, int32_t a0, int32_t na,
                                       double *dX, void *stream) {
   if (!ctx) return hfg::fail_external(HFG_INVALID_ARG, "hfg_mo_eri_ovov: null context");
+  if (const hfg_status st = hfg::ctx_select(ctx); st != HFG_OK) return st;
   Buffers buf;
   return transform(ctx, dC, i0, ni, a0, na, dX, static_cast<cudaStream_t>(stream), buf);
 }
@@ -267,6 +270,7 @@ extern "C" hfg_status hfg_mp2_rhf(hfg_ctx *ctx, const double *C, const double *e
   const int n = hfg_ctx_nbf(ctx);
   if (n <= 0 || nocc < 1 || nocc >= n) return hfg::fail_external(HFG_INVALID_ARG, "hfg_mp2_rhf: occupied count");
   const int nv = n - nocc;
+  if (const hfg_status st = hfg::ctx_select(ctx); st != HFG_OK) return st;
   Buffers buf;
   double *dC = nullptr, *dE = nullptr, *dX = nullptr, *dOut = nullptr;
   cudaError_t e = buf.get(&dC, (size_t)n * n);
@@ -323,6 +327,7 @@ extern "C" hfg_status hfg_mp2_uhf(hfg_ctx *ctx, const double *Cp, const double *
   if (n <= 0 || np < 0 || nm < 0 || np > n || nm > n)
     return hfg::fail_external(HFG_INVALID_ARG, "hfg_mp2_uhf: occupied counts (need 0 <= n+, n- <= nbf)");
   const int vp = n - np, vm = n - nm, lo = std::min(np, nm), hi = std::max(np, nm);
+  if (const hfg_status st = hfg::ctx_select(ctx); st != HFG_OK) return st;
   Buffers buf;
   double *dCp = nullptr, *dCm = nullptr, *dEp = nullptr, *dEm = nullptr, *dX = nullptr, *dOut = nullptr;
   const long long ovmax = std::max<long long>(1, std::max<long long>((long long)np * vp, (long long)nm * vm));
@@ -402,6 +407,7 @@ extern "C" hfg_status hfg_mo_eri_full(hfg_ctx *ctx, const double *dC, double *dX
   const int n = hfg_ctx_nbf(ctx);
   if (n <= 0) return hfg::fail_external(HFG_INVALID_ARG, "hfg_mo_eri_full: context without a single molecule");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (const hfg_status st = hfg::ctx_select(ctx); st != HFG_OK) return st;
   Buffers buf;
   MoTables t;
   hfg_status st = prepare(ctx, (long long)n * n, s, buf, t, who);
@@ -421,6 +427,7 @@ extern "C" hfg_status hfg_spin_orbital_eri(hfg_ctx *ctx, const double *C, double
   if (n <= 0) return hfg::fail_external(HFG_INVALID_ARG, "hfg_spin_orbital_eri: context without a single molecule");
   const long long m = 2LL * n, total = m * m * m * m, nn = (long long)n * n;
   if (count < total) return hfg::fail_external(HFG_INVALID_ARG, "hfg_spin_orbital_eri: output holds fewer than (2 nbf)^4");
+  if (const hfg_status st = hfg::ctx_select(ctx); st != HFG_OK) return st;
   Buffers buf;
   double *dC = nullptr, *dX = nullptr, *dT = nullptr;
   cudaError_t e = buf.get(&dC, (size_t)nn);

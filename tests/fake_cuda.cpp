@@ -97,7 +97,7 @@ void fake_clear() {
   bad.clear();
   log_.clear();
 }
-int fake_device() { return current; }
+void fake_set_device(int d) { current = d; }
 
 // --- registration
 void **__cudaRegisterFatBinary(void *) {

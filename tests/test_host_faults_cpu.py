@@ -108,7 +108,34 @@ def context_gives_everything_back(L):
     assert n > 10
 
 
-CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back)]
+def contexts_on_two_devices(L):
+    """Launches, buffers and handles belong to the context's device, whichever
+    one is current when it is called."""
+    os.environ["HFG_GROUP_MIN_TASKS"] = "0"
+    for path in ("0", "1"):
+        os.environ["HFG_WARP_PATH"] = path
+        for device in (0, 1):
+            Z, xyz = molecules.water_cluster(2, seed=1)
+            eng = E.Engine(Z, xyz, "6-31g*", device=device)
+            n = eng.nbf
+            P, C = np.eye(n), np.eye(n)
+            calls = [lambda: eng.set_prim_target(8), lambda: eng.fock_rhf(P), lambda: eng.fock_uhf(P, P),
+                     eng.eri_packed, lambda: eng.mp2_rhf(C, np.arange(n, dtype=float), 3),
+                     lambda: eng.mp2_uhf(C, np.arange(n, dtype=float), 3, C, np.arange(n, dtype=float), 2)]
+            for call in calls:
+                L.fake_set_device(1 - device)
+                call()
+                _sound(L)
+            small = E.Engine(*molecules.H2O_README, "sto-3g", device=device)
+            L.fake_set_device(1 - device)
+            small.spin_orbital_eri(np.eye(small.nbf))
+            _sound(L)
+            small.close()
+            eng.close()
+
+
+CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back,
+                              contexts_on_two_devices)]
 
 
 @pytest.mark.parametrize("case", CASES)
