@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(32 * group_warps(LA, LB, LC, LD), 1)
 #pragma unroll
       for (int x = 0; x < Cls::kAcc; ++x) acc[x] = 0.0;
       // far pass over all lanes, also those whose quartet is not far (replaced
-      // below) or not of the build (ignored).  The lanes of a group split the
-      // bra primitives, or the ket ones where those are too few.
+      // below) or not of the build (left out of the digestion).  The lanes of
+      // a group split the bra primitives, or the ket ones where those are too few.
       if (mon & ~nm) {
         const int G = 1 << lg;
         const bool bras = np >= G;
@@ -317,10 +317,6 @@ __global__ void __launch_bounds__(32 * group_warps(LA, LB, LC, LD), 1)
 #pragma unroll
           for (int d = 0; d < ND; ++d) dbd[sp][bb * ND + d] = __ldg(&Dm[sp][(aob + bb) * n + aod + d]);
         }
-      if (!on) {
-#pragma unroll
-        for (int x = 0; x < Cls::kAcc; ++x) acc[x] = 0.0;
-      }
 
       double out[N];
       Cls::template hrr<double>(out, acc, r.AB[0], r.AB[1], r.AB[2], Y0, Y1, Y2);
@@ -330,72 +326,76 @@ __global__ void __launch_bounds__(32 * group_warps(LA, LB, LC, LD), 1)
       const double s = on ? (bdiag ? 0.5 : 1.0) * (kdiag ? 0.5 : 1.0) * ((bdiag ? ~r.bp : r.bp) == kp ? 0.5 : 1.0) : 0.0;
       double jab[NA * NB];
 #pragma unroll
-      for (int a = 0; a < NA; ++a)
+      for (int x = 0; x < NA * NB; ++x) jab[x] = 0.0;
+      // a lane without a quartet of the build adds nothing, not even zero
+      // times a density entry that is not finite
+      if (s != 0.0) {
 #pragma unroll
-        for (int bb = 0; bb < NB; ++bb) {
-          const double nab = s * comp_norm<LA>(a) * comp_norm<LB>(bb);
-          const double dij = r.D[a * NB + bb];
-          double ja = 0.0;
+        for (int a = 0; a < NA; ++a)
 #pragma unroll
-          for (int c = 0; c < NC; ++c)
+          for (int bb = 0; bb < NB; ++bb) {
+            const double nab = s * comp_norm<LA>(a) * comp_norm<LB>(bb);
+            const double dij = r.D[a * NB + bb];
+            double ja = 0.0;
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+#pragma unroll
+              for (int d = 0; d < ND; ++d) {
+                const int x = ((a * NB + bb) * NC + c) * ND + d;
+                out[x] *= nab * comp_norm<LC>(c) * comp_norm<LD>(d);
+                ja += out[x] * __ldg(&DJ[(aoc + c) * n + aod + d]);
+                jcd[c * ND + d] += out[x] * dij;
+              }
+            jab[a * NB + bb] = 2.0 * ja;
+          }
+#pragma unroll
+        for (int sp = 0; sp < NS; ++sp) {
+          double *K = Km[sp];
+          // K_ac += (ab|cd) D_bd, K_ad += (ab|cd) D_bc
+#pragma unroll
+          for (int bb = 0; bb < NB; ++bb) {
 #pragma unroll
             for (int d = 0; d < ND; ++d) {
-              const int x = ((a * NB + bb) * NC + c) * ND + d;
-              out[x] *= nab * comp_norm<LC>(c) * comp_norm<LD>(d);
-              ja += out[x] * __ldg(&DJ[(aoc + c) * n + aod + d]);
-              jcd[c * ND + d] += out[x] * dij;
+              const double x = dbd[sp][bb * ND + d];
+#pragma unroll
+              for (int a = 0; a < NA; ++a)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) kac[sp][a * NC + c] += out[((a * NB + bb) * NC + c) * ND + d] * x;
             }
-          jab[a * NB + bb] = 2.0 * ja;
-        }
 #pragma unroll
-      for (int sp = 0; sp < NS; ++sp) {
-        double *K = Km[sp];
-        // K_ac += (ab|cd) D_bd, K_ad += (ab|cd) D_bc
+            for (int c = 0; c < NC; ++c) {
+              const double x = dbc[sp][bb * NC + c];
 #pragma unroll
-        for (int bb = 0; bb < NB; ++bb) {
+              for (int a = 0; a < NA; ++a)
 #pragma unroll
-          for (int d = 0; d < ND; ++d) {
-            const double x = dbd[sp][bb * ND + d];
-#pragma unroll
-            for (int a = 0; a < NA; ++a)
-#pragma unroll
-              for (int c = 0; c < NC; ++c) kac[sp][a * NC + c] += out[((a * NB + bb) * NC + c) * ND + d] * x;
+                for (int d = 0; d < ND; ++d) kad[sp][a * ND + d] += out[((a * NB + bb) * NC + c) * ND + d] * x;
+            }
           }
+          // K_bc += (ab|cd) D_ad, K_bd += (ab|cd) D_ac
+          double kbc[NB * NC], kbd[NB * ND];
 #pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            const double x = dbc[sp][bb * NC + c];
+          for (int x = 0; x < NB * NC; ++x) kbc[x] = 0.0;
 #pragma unroll
-            for (int a = 0; a < NA; ++a)
+          for (int x = 0; x < NB * ND; ++x) kbd[x] = 0.0;
 #pragma unroll
-              for (int d = 0; d < ND; ++d) kad[sp][a * ND + d] += out[((a * NB + bb) * NC + c) * ND + d] * x;
+          for (int a = 0; a < NA; ++a) {
+#pragma unroll
+            for (int d = 0; d < ND; ++d) {
+              const double x = __ldg(&Dm[sp][(aoa + a) * n + aod + d]);
+#pragma unroll
+              for (int bb = 0; bb < NB; ++bb)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) kbc[bb * NC + c] += out[((a * NB + bb) * NC + c) * ND + d] * x;
+            }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              const double x = __ldg(&Dm[sp][(aoa + a) * n + aoc + c]);
+#pragma unroll
+              for (int bb = 0; bb < NB; ++bb)
+#pragma unroll
+                for (int d = 0; d < ND; ++d) kbd[bb * ND + d] += out[((a * NB + bb) * NC + c) * ND + d] * x;
+            }
           }
-        }
-        // K_bc += (ab|cd) D_ad, K_bd += (ab|cd) D_ac
-        double kbc[NB * NC], kbd[NB * ND];
-#pragma unroll
-        for (int x = 0; x < NB * NC; ++x) kbc[x] = 0.0;
-#pragma unroll
-        for (int x = 0; x < NB * ND; ++x) kbd[x] = 0.0;
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-#pragma unroll
-          for (int d = 0; d < ND; ++d) {
-            const double x = __ldg(&Dm[sp][(aoa + a) * n + aod + d]);
-#pragma unroll
-            for (int bb = 0; bb < NB; ++bb)
-#pragma unroll
-              for (int c = 0; c < NC; ++c) kbc[bb * NC + c] += out[((a * NB + bb) * NC + c) * ND + d] * x;
-          }
-#pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            const double x = __ldg(&Dm[sp][(aoa + a) * n + aoc + c]);
-#pragma unroll
-            for (int bb = 0; bb < NB; ++bb)
-#pragma unroll
-              for (int d = 0; d < ND; ++d) kbd[bb * ND + d] += out[((a * NB + bb) * NC + c) * ND + d] * x;
-          }
-        }
-        if (s != 0.0) {
 #pragma unroll
           for (int bb = 0; bb < NB; ++bb) {
 #pragma unroll
