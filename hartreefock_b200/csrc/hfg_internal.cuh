@@ -106,18 +106,25 @@ __host__ __device__ constexpr int group_warps(int la, int lb, int lc, int ld) {
 // warp-cooperative kernel, a quartet per warp, instead of the split path, a
 // quartet per thread: the thread takes 50 to 300 us over one quartet however
 // few there are, the warp a fraction of that, until there are enough to fill
-// the GPU with threads.  The lines are where the two meet (us per J/K build of
-// (H2O)2, 4, 8, 12, 16 / 6-31G*, warp kernel against split path): (dd|dp) 45, 45,
-// 66, 125, 273 against 286, 292, 315, 351, 432 (9,074 primitive quartets in the
-// last); (dd|pp) 50, 51, 95, 164, 271 against 111, 139, 130, 165, 172 (9,019 in
-// (H2O)12); (dd|ds) 39, 43, 93 against 59, 77, 87 (5,523 in (H2O)8); (dd|ps) 56, 54,
-// 156 against 52, 58, 69 (4,541 in (H2O)4); (dp|pp) 78, 109 against 94, 104 (3,994 in
-// (H2O)4); (dp|ds) is level at 470.  (dd|dd) is faster here at every size (0.24
-// against 0.82 ms at (H2O)16, before its recursions became tables).  (dp|dp) would
-// gain too (56 against 157 at (H2O)2), but this kernel is 3.1e-12 off the
-// reference on two cancelling elements of O2 / 6-31G* (1.3e-12 on the split path;
-// adding the transfer terms one by one as the per-thread code does changes
-// nothing), so it stays where it was.
+// the GPU with threads.  us per J/K build, warp kernel against split path, at
+// the primitive quartets of (H2O)1 to (H2O)24 / 6-31G* and C2H6 to C9H20:
+//   (dd|dp)  43/264 at 4, 66/309 at 2,106, 127/356 at 6,078, 228/405 at 12,186,
+//            273/432 at 16,640, 437/551 at 28,666, level at 40,104: 16,000 is
+//            below where they meet
+//   (dd|pp)  50/87 at 13, 93/128 at 4,844, 146/159 at 9,506, 162/166 at 14,313,
+//            269/173 at 36,401
+//   (dd|ds)  37/48 at 18, 50/77 at 2,405, 78/81 at 3,866, 93/88 at 8,367
+//   (dp|pp)  78/89 at 52, 80/96 at 1,994, 109/98 at 4,836
+//   (dd|ps)  52/49 at 72, 56/54 at 550, level at 1,014 and 2,167, 54/57 at 5,169,
+//            82/58 at 8,514; the one launch instead of two decides it in whole
+//            builds on class streams: 170/204 at 184 (CH3), 265/280 at 1,014
+//            (C2H6), 277/288 at 2,167 ((H2O)3), 382/311 at 5,169 ((H2O)4)
+//   (dp|ds)  60/57 at 72, 70/65 at 3,574, 89/65 at 8,730: the split path
+// (dd|dd) is faster here at every size (0.24 against 0.82 ms at (H2O)16, before
+// its recursions became tables).  (dp|dp) would gain too (56 against 161 at
+// (H2O)2), but this kernel is 3.1e-12 off the reference on two cancelling
+// elements of O2 / 6-31G* (1.3e-12 on the split path; adding the transfer terms
+// one by one as the per-thread code does changes nothing), so it stays there.
 __host__ __device__ constexpr long long warp_prim_limit(int la, int lb, int lc, int ld) {
   const int ket = 10 * lc + ld;
   if (la == 2 && lb == 2)

@@ -364,9 +364,10 @@ hfg_status hfg_autotune_tasks(hfg_ctx *ctx, const double *dP, int32_t *chosen, i
  * (one warp per shell quartet, recursions from a level-ordered program in
  * shared memory, no scratch), 0 on the split path (primitive kernel, then the
  * HRR / digestion kernel over scratch).  Default: warp for (dd|dd) and, but
- * for (dp|dp), (dp|ds) and mixed-precision builds, for the classes with few
- * primitive quartets; split for the rest.  HFG_INVALID_ARG for a class without both kernels.  Batched
- * asynchronous builds and hfg_fock_rhf_noalloc always use the warp kernel. */
+ * for mixed-precision builds, for (dd|dp), (dd|pp), (dd|ds), (dd|ps) and (dp|pp)
+ * with few primitive quartets; split for the rest.  HFG_INVALID_ARG for a class without
+ * both kernels.  Batched asynchronous builds and hfg_fock_rhf_noalloc always
+ * use the warp kernel. */
 hfg_status hfg_set_class_path(hfg_ctx *ctx, int32_t la, int32_t lb, int32_t lc, int32_t ld, int32_t path);
 /* Picks that kernel per class by timing both on the caller's device density
  * dP (one warm-up, two timed launches each, CUDA events); `chosen` receives
