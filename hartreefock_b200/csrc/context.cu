@@ -194,6 +194,7 @@ struct hfg_ctx {
   int prim_target = 96;
   int class_prim_target[kNumClasses] = {};
   int group_min_tasks = kGroupMinTasks;  // HFG_GROUP_MIN_TASKS
+  int group_run = 0;  // most bras of a grouped task (HFG_GROUP_RUN); 0 = by the class's tasks
   // CUDA graph of the plain direct build (hfg_set_graphs): captured on the
   // second build with the same buffers, stream and settings, replayed after
   bool use_graphs = false;
@@ -425,7 +426,8 @@ static void build_group_tasks(const hfg_ctx *c, QuartetClass &q, const std::vect
   const PairClassList &BL = c->pclass[q.bra_pc], &KL = c->pclass[q.ket_pc];
   const auto &bras = BL.gpairs;
   // bras per task: as many as leave several tasks for every warp of the GPU
-  const int most = (int)std::max<int64_t>(1, std::min<int64_t>(kGroupMaxBras, (int64_t)q.tasks.size() / (kGroupSms * 96)));
+  const int64_t wanted = c->group_run > 0 ? c->group_run : (int64_t)q.tasks.size() / (kGroupSms * 96);
+  const int most = (int)std::max<int64_t>(1, std::min<int64_t>(kGroupMaxBras, wanted));
   q.gtasks.clear();
   q.gcost_prefix.assign(1, 0.0);
   q.ngmasks = 0;
@@ -1652,6 +1654,8 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
   if (const char *e = std::getenv("HFG_BLOCKS_PER_SM")) ctx->blocks_per_sm = std::max(1, std::atoi(e));
   // tuning: HFG_GROUP_MIN_TASKS sets the tasks per SM from which a class runs the grouped kernel
   if (const char *e = std::getenv("HFG_GROUP_MIN_TASKS")) ctx->group_min_tasks = std::max(0, std::atoi(e));
+  // tuning: HFG_GROUP_RUN sets the most bras of a grouped task (1 .. 16)
+  if (const char *e = std::getenv("HFG_GROUP_RUN")) ctx->group_run = std::max(0, std::atoi(e));
   // tuning: HFG_PRIM_TARGET sets the lane-group target (0: one lane per quartet)
   if (const char *e = std::getenv("HFG_PRIM_TARGET")) ctx->prim_target = std::max(0, std::atoi(e));
   // default kernel per large class: by its primitive quartets (warp_prim_limit);
@@ -2141,7 +2145,8 @@ hfg_status hfg_class_profile(const hfg_ctx *c, hfg_class_time *out, int32_t cap,
     const ClassEntry &e = kClasses[q.cls];
     out[n] = hfg_class_time{e.la,    e.lb,    e.lc,         e.ld, q.shell_quartets, q.function_quartets, q.prim_quartets,
                             q.flops, (double)q.last_ms, (int64_t)q.tasks.size(),
-                            q.warp_work > 0 ? q.lane_work / q.warp_work : 0.0, class_on_warp(c, q.cls, c->mixed_cutoff > 0 ? 2 : 0) ? 1 : 0, 0};
+                            q.warp_work > 0 ? q.lane_work / q.warp_work : 0.0, class_on_warp(c, q.cls, c->mixed_cutoff > 0 ? 2 : 0) ? 1 : 0,
+                            !c->precision_form() && uses_group(c, q) ? 1 : 0};
     ++n;
   }
   *count = n;

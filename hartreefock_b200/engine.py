@@ -67,7 +67,7 @@ class hfg_class_time(ctypes.Structure):
                 ("shell_quartets", ctypes.c_int64), ("function_quartets", ctypes.c_int64),
                 ("primitive_quartets", ctypes.c_int64), ("flops", ctypes.c_double), ("ms", ctypes.c_double),
                 ("tasks", ctypes.c_int64), ("lane_occupancy", ctypes.c_double), ("warp_kernel", ctypes.c_int32),
-                ("reserved", ctypes.c_int32)]
+                ("grouped", ctypes.c_int32)]
 
 
 _lib = None

@@ -404,7 +404,7 @@ typedef struct {
   double lane_occupancy;    /* primitive quartets the lanes evaluate / (32 x the longest
                                lane loop) over the tasks, for a thread per quartet */
   int32_t warp_kernel;      /* 1: one warp per quartet (the large classes) */
-  int32_t reserved;
+  int32_t grouped;          /* 1: runs of bras share a ket chunk (light classes of large molecules) */
 } hfg_class_time;
 hfg_status hfg_set_profiling(hfg_ctx *ctx, int32_t on);
 /* Writes up to `cap` entries (largest flops first); *count = entries written. */

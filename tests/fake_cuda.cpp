@@ -79,6 +79,29 @@ void use(const void *p, size_t bytes, const std::string &what) {
   if (capturing) captured.push_back(u);
   check(u);
 }
+
+// Entries of the allocation from p on.
+template <class T>
+long long entries(const T *p) {
+  const char *q = reinterpret_cast<const char *>(p);
+  auto it = blocks.upper_bound(q);
+  if (it == blocks.begin()) return 0;
+  --it;
+  return (it->first + it->second.bytes - q) / (long long)sizeof(T);
+}
+int longest_run = 0;
+// Every range of a grouped launch's tasks lies in its lists.
+void check_group_tasks(const hfg::ClassLaunch &cl, const std::string &name) {
+  if (cl.ntasks_dev || entries(cl.tasks) < cl.task_offset + cl.ntasks) return;
+  for (int t = cl.task_offset; t < cl.task_offset + cl.ntasks; ++t) {
+    const hfg::GroupTask g = hfg::group_task(cl.tasks[t]);
+    longest_run = std::max(longest_run, g.nbra);
+    if (g.nbra < 1 || g.nbra > hfg::kGroupMaxBras || g.nket < 1 || g.nket << g.lg > 32 ||
+        g.bra_start + g.nbra > entries(cl.bra_list) || g.ket_start + g.nket > entries(cl.ket_list) ||
+        (long long)g.mask_off + g.nbra > entries(cl.masks))
+      complain(name + ": task outside its lists");
+  }
+}
 }  // namespace
 
 extern "C" {
@@ -92,6 +115,11 @@ long long fake_peak_bytes(int restart) {
   return (long long)peak_live;
 }
 const char *fake_complaints() { return bad.c_str(); }
+int fake_longest_run() {
+  const int r = longest_run;
+  longest_run = 0;
+  return r;
+}
 const char *fake_log() { return log_.c_str(); }
 void fake_clear() {
   bad.clear();
@@ -300,6 +328,7 @@ cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **args, size_t smem
       use(cl.masks, sizeof(uint2), name + " masks");
       use(cl.ket_blocks, kKetStride * sizeof(double), name + " ket blocks");
       use(cl.ket_block_off, 4, name + " ket block offsets");
+      check_group_tasks(cl, name);
     }
   } else if (has("group_masks_kernel")) {
     for (int a : {1, 2, 3, 4, 9}) use(*static_cast<void **>(args[a]), 4, name + " argument " + std::to_string(a));

@@ -134,8 +134,29 @@ def contexts_on_two_devices(L):
             eng.close()
 
 
+def grouped_runs(L):
+    """The runs of the grouped tasks are as long as asked for, inside their lists."""
+    Z, xyz = molecules.water_cluster(4, seed=1)
+    os.environ["HFG_GROUP_MIN_TASKS"] = "0"
+    for run, least, most in ((1, 1, 1), (3, 3, 3), (16, 8, 16), (100, 8, 16)):
+        os.environ["HFG_GROUP_RUN"] = str(run)
+        eng = E.Engine(Z, xyz, "6-31g*")
+        for target in (0, 8, 96):
+            eng.set_prim_target(target)
+            eng.fock_rhf(np.eye(eng.nbf))
+            assert least <= L.fake_longest_run() <= most
+            assert sum(c["grouped"] for c in eng.class_profile()) == 8
+        _sound(L)
+        eng.close()
+    # small molecules are not grouped of themselves
+    del os.environ["HFG_GROUP_MIN_TASKS"]
+    eng = E.Engine(Z, xyz, "6-31g*")
+    eng.fock_rhf(np.eye(eng.nbf))
+    assert L.fake_longest_run() == 0 and not any(c["grouped"] for c in eng.class_profile())
+
+
 CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back,
-                              contexts_on_two_devices)]
+                              contexts_on_two_devices, grouped_runs)]
 
 
 @pytest.mark.parametrize("case", CASES)
