@@ -173,7 +173,8 @@ struct hfg_ctx {
   PairClassList pclass[kNumPairClasses];
   std::vector<QuartetClass> qclasses;
   bool lists_ready = false;   // qclasses and their device lists are complete
-  bool group_layout = false;  // so is what upload_group_layout makes
+  bool groups_made = false;   // the grouped lists of the classes above the line too
+  bool group_layout = false;  // and what upload_group_layout makes
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // class kernels of one build are independent (J/K by atomics): they run on
@@ -275,6 +276,8 @@ struct hfg_ctx {
   // handle), destroyed with the context
   void *handle = nullptr;
   void (*handle_destroy)(void *) = nullptr;
+  // grouped lists serve plain builds only
+  bool wants_groups() const { return batch || !precision_form(); }
   bool precision_form() const { return opts.density_screening || opts.incremental || mixed_cutoff > 0; }
   double density_threshold() const {
     return opts.density_threshold > 0 ? opts.density_threshold : opts.schwarz_threshold;
@@ -416,21 +419,48 @@ static inline int64_t pair_functions(const hfg_ctx *c, int p) {
 // sharded build makes the same lists.
 constexpr int kGroupSms = 148;
 
-// Grouped tasks of one class (eri_group.cuh): every run of bras with one first
-// shell (same molecule and primitive bucket) against every chunk of kets of a
-// bucket that one of them reaches.  `ends`: per bra position and ket bucket the
-// end of the bra's kets, -1 for none.
-static void build_group_tasks(const hfg_ctx *c, QuartetClass &q, const std::vector<int> &ends,
-                              const std::vector<int> &segmax, const std::vector<int64_t> &kprim, int target,
-                              double prim_cost, double quartet_cost) {
+// The longest contraction of each bucket segment of a pair class.
+static std::vector<int> segment_prims(const hfg_ctx *c, const PairClassList &L) {
+  std::vector<int> most(L.seg_start.size(), 0);
+  for (size_t g = 0; g + 1 < L.seg_start.size(); ++g)
+    for (int k = L.seg_start[g]; k < L.seg_start[g + 1]; ++k) most[g] = std::max(most[g], c->pair_nprim[L.pairs[k]]);
+  return most;
+}
+
+// Primitive quartets per lane that the class's tasks aim for (0: one lane per quartet).
+static int lane_target(const hfg_ctx *c, int cls) {
+  return c->class_prim_target[cls] > 0 ? c->class_prim_target[cls] : c->class_prim_target[cls] < 0 ? 0 : c->prim_target;
+}
+
+// flops of one primitive quartet of a class with its Boys function
+static double primitive_cost(const hfg_ctx *c, int cls) {
+  const ClassEntry &e = kClasses[cls];
+  return prim_flops(cls, c->opts.eri_convention == HFG_ERI_REFERENCE) + boys_geom_flops(e.la + e.lb + e.lc + e.ld);
+}
+
+// Grouped tasks of one class (eri_group.cuh), from its list of tasks with one
+// bra each: every run of bras with one first shell (same molecule and primitive
+// bucket) against every chunk of kets of a bucket that one of them reaches.
+// None below the line (kGroupMinTasks).
+static void build_group_tasks(const hfg_ctx *c, QuartetClass &q) {
+  if (!kGroup[q.cls] || (int64_t)q.tasks.size() < (int64_t)c->group_min_tasks * kGroupSms) return;
   const PairClassList &BL = c->pclass[q.bra_pc], &KL = c->pclass[q.ket_pc];
+  const int target = lane_target(c, q.cls);
+  const double prim_cost = primitive_cost(c, q.cls), quartet_cost = hrr_flops(q.cls);
+  const std::vector<int> segmax = segment_prims(c, KL);
+  std::vector<int64_t> kprim(KL.pairs.size() + 1, 0);
+  for (size_t k = 0; k < KL.pairs.size(); ++k) kprim[k + 1] = kprim[k] + c->pair_nprim[KL.pairs[k]];
+  // per bra position and ket bucket the end of the bra's kets, -1 for none
+  std::vector<int> ends(BL.pairs.size() * kBuckets, -1);
+  for (const Task &t : q.tasks) {
+    int &e = ends[(size_t)t.bra_pos * kBuckets + prim_bucket(c->pair_nprim[KL.pairs[t.ket_start]])];
+    e = std::max(e, t.ket_end);
+  }
   const auto &bras = BL.gpairs;
   // bras per task: as many as leave several tasks for every warp of the GPU
   const int64_t wanted = c->group_run > 0 ? c->group_run : (int64_t)q.tasks.size() / (kGroupSms * 96);
   const int most = (int)std::max<int64_t>(1, std::min<int64_t>(kGroupMaxBras, wanted));
-  q.gtasks.clear();
   q.gcost_prefix.assign(1, 0.0);
-  q.ngmasks = 0;
   // long contractions first, so that the light tasks fill the end of the launch
   std::vector<size_t> order;
   for (int k = kBuckets - 1; k >= 0; --k)
@@ -503,24 +533,16 @@ static QuartetClass build_quartet_class(const hfg_ctx *c, int ci, double thresho
     kprim[k + 1] = kprim[k] + c->pair_nprim[kets[k]];
     kq[k] = c->pair_Q[kets[k]];
   }
-  const double pf = prim_flops(ci, c->opts.eri_convention == HFG_ERI_REFERENCE);
+  const double pf = primitive_cost(c, ci);
   const double hf = hrr_flops(ci);
-  const int ltot = ce.la + ce.lb + ce.lc + ce.ld;
-  // the longest ket contraction of each bucket segment
-  std::vector<int> segmax(KL.seg_start.size(), 0);
-  for (size_t g = 0; g + 1 < KL.seg_start.size(); ++g)
-    for (int64_t k2 = KL.seg_start[g]; k2 < KL.seg_start[g + 1]; ++k2)
-      segmax[g] = std::max(segmax[g], c->pair_nprim[kets[k2]]);
+  const std::vector<int> segmax = segment_prims(c, KL);  // of the kets
   // fused thread-per-quartet classes: lanes per quartet so that a lane's
   // share of a quartet's primitive quartets stays near the target (long
   // contractions spread over 2..32 lanes, fewer kets per task); the large
   // classes (split path: one lane per quartet; warp kernel: one warp per
   // quartet) keep 32 kets per task
   const bool grouped = !kSplit[ci] && !kWarp[ci];
-  // per bra and ket bucket: the end of its kets (grouped tasks)
-  std::vector<int> ends(kGroup[ci] ? bras.size() * kBuckets : 0, -1);
-  const int target = c->class_prim_target[ci] > 0 ? c->class_prim_target[ci]
-                     : c->class_prim_target[ci] < 0 ? 0 : c->prim_target;
+  const int target = lane_target(c, ci);
   for (size_t b = 0; b < bras.size(); ++b) {
     const double qb = c->pair_Q[bras[b]];
     if (!(qb > 0)) continue;
@@ -541,7 +563,6 @@ static QuartetClass build_quartet_class(const hfg_ctx *c, int ci, double thresho
       int64_t end = lo;
       if (same) end = std::min<int64_t>(end, (int64_t)b + 1);
       if (end <= s0) continue;
-      if (kGroup[ci]) ends[b * kBuckets + k] = (int)end;
       int per_task = 32;
       if (grouped && target > 0) {
         const double work = (double)bprim * segmax[mol * kBuckets + k];
@@ -563,7 +584,7 @@ static QuartetClass build_quartet_class(const hfg_ctx *c, int ci, double thresho
         q.warp_work += 32.0 * std::ceil((double)bprim * (double)mx / (double)(1 << tk.lg));
         if (q.cost_prefix.empty()) q.cost_prefix.push_back(0.0);
         q.cost_prefix.push_back(q.cost_prefix.back() +
-                                (double)bprim * (double)(kprim[e1] - kprim[st]) * (pf + boys_geom_flops(ltot)) +
+                                (double)bprim * (double)(kprim[e1] - kprim[st]) * pf +
                                 (double)(e1 - st) * hf);
       }
       q.shell_quartets += end - s0;
@@ -576,16 +597,13 @@ static QuartetClass build_quartet_class(const hfg_ctx *c, int ci, double thresho
       q.prim_quartets += bprim * (kprim[end] - kprim[s0]);
     }
   }
-  q.flops = (double)q.prim_quartets * (pf + boys_geom_flops(ltot)) + (double)q.shell_quartets * hf;
-  if (kGroup[ci] && (int64_t)q.tasks.size() >= (int64_t)c->group_min_tasks * kGroupSms)
-    build_group_tasks(c, q, ends, segmax, kprim, target, pf + boys_geom_flops(ltot), hf);
+  q.flops = (double)q.prim_quartets * pf + (double)q.shell_quartets * hf;
+  if (c->wants_groups()) build_group_tasks(c, q);
   return q;
 }
 
-static void build_quartet_classes(hfg_ctx *c, double threshold) {
-  c->qclasses.clear();
-  std::fill(std::begin(c->class_prims), std::end(c->class_prims), int64_t(0));
-  // bra order of the grouped tasks
+// bra order of the grouped tasks
+static void order_group_bras(hfg_ctx *c) {
   for (PairClassList &L : c->pclass) {
     if (L.gpairs.size() == L.pairs.size()) continue;
     L.gpairs = L.pairs;
@@ -593,13 +611,22 @@ static void build_quartet_classes(hfg_ctx *c, double threshold) {
       std::stable_sort(L.gpairs.begin() + L.seg_start[x], L.gpairs.begin() + L.seg_start[x + 1],
                        [&](int a, int b) { return c->pair_sa[a] < c->pair_sa[b]; });
   }
-  // the classes' lists are independent: one thread each for large molecules
-  // ((H2O)32 / 6-31G*: 3.2 million tasks)
+}
+
+// One thread per class for large molecules ((H2O)32 / 6-31G*: 3.2 million
+// tasks), or the calling one, where no thread is to be had.
+static std::launch list_threads(const hfg_ctx *c) {
+  return c->npairs >= 4096 ? std::launch::async | std::launch::deferred : std::launch::deferred;
+}
+
+static void build_quartet_classes(hfg_ctx *c, double threshold) {
+  c->qclasses.clear();
+  std::fill(std::begin(c->class_prims), std::end(c->class_prims), int64_t(0));
+  if (c->wants_groups()) order_group_bras(c);
+  // the classes' lists are independent
   std::vector<std::future<QuartetClass>> lists;
-  // (or on this one, where no thread is to be had)
-  const auto how = c->npairs >= 4096 ? std::launch::async | std::launch::deferred : std::launch::deferred;
   for (int ci = 0; ci < kNumClasses; ++ci)
-    lists.push_back(std::async(how, [c, ci, threshold] { return build_quartet_class(c, ci, threshold); }));
+    lists.push_back(std::async(list_threads(c), [c, ci, threshold] { return build_quartet_class(c, ci, threshold); }));
   for (int ci = 0; ci < kNumClasses; ++ci) {
     QuartetClass q = lists[ci].get();
     c->class_prims[ci] = q.prim_quartets;
@@ -694,12 +721,10 @@ static hfg_status make_group_layout(hfg_ctx *c) {
   if ((st = upload(&c->d_pair_pos, c->pair_pos)) != HFG_OK) return st;
   for (PairClassList &L : c->pclass) {
     if (L.pairs.empty()) continue;
+    const std::vector<int> of_segment = segment_prims(c, L);
     std::vector<int> segmax(L.pairs.size(), 0), off, records;
-    for (size_t x = 0; x + 1 < L.seg_start.size(); ++x) {
-      int most = 0;
-      for (int k = L.seg_start[x]; k < L.seg_start[x + 1]; ++k) most = std::max(most, c->pair_nprim[L.pairs[k]]);
-      std::fill(segmax.begin() + L.seg_start[x], segmax.begin() + L.seg_start[x + 1], most);
-    }
+    for (size_t x = 0; x + 1 < L.seg_start.size(); ++x)
+      std::fill(segmax.begin() + L.seg_start[x], segmax.begin() + L.seg_start[x + 1], of_segment[x]);
     int total = 0;
     for (size_t x = 0; x < L.pairs.size(); x += 32) {
       // as many records as the longest contraction of a segment the block
@@ -743,14 +768,14 @@ static hfg_status need_lists(const hfg_ctx *c) {
                                                  "(hfg_set_prim_target tries again)");
 }
 
-static hfg_status upload_classes(hfg_ctx *c) {
+// The grouped lists' device copies and ket masks, after the tasks'.
+static hfg_status upload_groups(hfg_ctx *c) {
   for (const auto &q : c->qclasses)
     if (!q.gtasks.empty())
       if (const hfg_status st = upload_group_layout(c); st != HFG_OK) return st;
   for (auto &q : c->qclasses) {
-    hfg_status st = upload(&q.d_tasks, q.tasks);
-    if (st != HFG_OK || (st = upload(&q.d_gtasks, q.gtasks)) != HFG_OK) return st;
     if (q.gtasks.empty()) continue;
+    if (const hfg_status st = upload(&q.d_gtasks, q.gtasks); st != HFG_OK) return st;
     HFG_CUDA(cudaMalloc((void **)&q.d_gmasks, q.ngmasks * sizeof(uint2)));
     const ClassEntry &e = kClasses[q.cls];
     const int grid = std::max(1, std::min(c->num_sms * 8, ((int)q.gtasks.size() + 7) / 8));
@@ -760,8 +785,38 @@ static hfg_status upload_classes(hfg_ctx *c) {
     HFG_CUDA(cudaGetLastError());
   }
   HFG_CUDA(cudaStreamSynchronize(c->stream));
+  c->groups_made = true;
+  return HFG_OK;
+}
+
+static hfg_status upload_classes(hfg_ctx *c) {
+  for (auto &q : c->qclasses)
+    if (const hfg_status st = upload(&q.d_tasks, q.tasks); st != HFG_OK) return st;
+  if (c->wants_groups())
+    if (const hfg_status st = upload_groups(c); st != HFG_OK) return st;
   c->lists_ready = true;
   return HFG_OK;
+}
+
+// The grouped lists of a context that was in the precision form when its tasks
+// were listed, whose builds have no use for them, before its first plain build.
+static hfg_status ensure_groups(hfg_ctx *c) {
+  if (c->groups_made) return HFG_OK;
+  order_group_bras(c);
+  std::vector<std::future<void>> lists;
+  for (auto &q : c->qclasses) lists.push_back(std::async(list_threads(c), [c, &q] { build_group_tasks(c, q); }));
+  for (auto &l : lists) l.get();
+  const hfg_status st = upload_groups(c);
+  if (st != HFG_OK)
+    for (auto &q : c->qclasses) {
+      cudaFree(q.d_gtasks);
+      cudaFree(q.d_gmasks);
+      q.d_gtasks = nullptr;
+      q.d_gmasks = nullptr;
+      q.gtasks.clear();
+      q.ngmasks = 0;
+    }
+  return st;
 }
 
 // blocks of a fused class launch: one warp per task, fused_warps() per block
@@ -1230,6 +1285,8 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
 static hfg_status direct_build(hfg_ctx *c, bool uhf, const double *dPa, const double *dPb, double *dGa, double *dGb,
                                cudaStream_t s) {
   if (const hfg_status st = need_lists(c); st != HFG_OK) return st;
+  if (!c->precision_form())
+    if (const hfg_status st = ensure_groups(c); st != HFG_OK) return st;
   const bool graphable = c->use_graphs && !c->batch && !c->precision_form() && !c->profiling && s != nullptr &&
                          s != cudaStreamLegacy && s != cudaStreamPerThread;
   if (!graphable) return direct_build_body(c, uhf, dPa, dPb, dGa, dGb, s, false);
@@ -2334,7 +2391,7 @@ static void free_classes(hfg_ctx *c) {
   c->d_task_counts = nullptr;
   c->d_queue = nullptr;
   c->task_base.clear();
-  c->lists_ready = false;
+  c->lists_ready = c->groups_made = false;
   ++c->config_version;  // a captured graph holds the freed lists
 }
 

@@ -155,8 +155,46 @@ def grouped_runs(L):
     assert L.fake_longest_run() == 0 and not any(c["grouped"] for c in eng.class_profile())
 
 
+def precision_contexts_hold_no_grouped_lists(L):
+    """Contexts in the precision form hold the lists their builds read; the
+    first plain build makes the grouped ones, whole or not at all."""
+    Z, xyz = molecules.water_cluster(3, seed=1)
+    P = np.eye(57)
+
+    def held(min_tasks, **options):
+        os.environ["HFG_GROUP_MIN_TASKS"] = min_tasks
+        start = L.fake_live_bytes()
+        eng = E.Engine(Z, xyz, "6-31g*", **options)
+        return eng, L.fake_live_bytes() - start
+
+    for options in ({"incremental": True}, {"mixed_cutoff": 1e-4}, {"density_screening": True}):
+        assert held("0", **options)[1] == held("1000000000", **options)[1]
+    assert held("0")[1] > held("1000000000")[1]
+    for n in range(1, 100):
+        eng, _ = held("0", incremental=True)
+        eng.set_graphs(True)
+        eng.fock_rhf(P)
+        eng.set_incremental(False)
+        L.fake_fail_allocation(n)
+        try:
+            eng.fock_rhf(P)
+            failed = False
+        except E.HfgError:
+            failed = True
+        L.fake_fail_allocation(0)
+        for _ in range(3):
+            eng.fock_rhf(P)
+        assert sum(c["grouped"] for c in eng.class_profile()) == 8 and L.fake_longest_run() > 0
+        _sound(L)
+        eng.close()
+        if not failed:
+            break
+    assert n > 10
+
+
 CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back,
-                              contexts_on_two_devices, grouped_runs)]
+                              contexts_on_two_devices, grouped_runs,
+                              precision_contexts_hold_no_grouped_lists)]
 
 
 @pytest.mark.parametrize("case", CASES)
