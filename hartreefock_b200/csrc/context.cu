@@ -1097,6 +1097,7 @@ static hfg_status grow_scratch(hfg_ctx *c, int slot, size_t need) {
   return HFG_OK;
 }
 
+static hfg_status ensure_queue(hfg_ctx *c);
 static hfg_status ensure_task_scratch(hfg_ctx *c);
 __global__ void compact_screened_tasks(const EngineView v, const ClassLaunch cl, Task *__restrict__ out, int *count);
 
@@ -1195,7 +1196,7 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
   bool grouped = false;
   for (const QuartetClass &q : c->qclasses) grouped = grouped || (!precise && uses_group(c, q));
   if ((c->use_queue || compact || grouped) && nq > 0) {
-    if ((st = ensure_task_scratch(c)) != HFG_OK) return st;
+    if ((st = compact ? ensure_task_scratch(c) : ensure_queue(c)) != HFG_OK) return st;
     HFG_CUDA(cudaMemsetAsync(c->d_queue, 0, nq * sizeof(int), s));
     ++launches;
     if (compact) {
@@ -1356,11 +1357,14 @@ __global__ void finalize_uhf_batch(const double *J, const double *Ka, const doub
   }
 }
 
-// Tasks of active molecules, in the class's order up to warp-sized groups:
-// each warp writes its kept tasks as one contiguous run (ballot + one
-// atomic per warp).
+// Work-queue counters, one per quartet class.
+static hfg_status ensure_queue(hfg_ctx *c) {
+  if (!c->d_queue) HFG_CUDA(cudaMalloc((void **)&c->d_queue, std::max<size_t>(1, c->qclasses.size()) * sizeof(int)));
+  return HFG_OK;
+}
+
 // Device lists of compacted tasks (one region per quartet class, as long as
-// the class's task list), their counts and work-queue counters; allocated by
+// the class's task list), their counts and the work-queue counters; allocated by
 // the first build that compacts, freed when the task lists are rebuilt.
 static hfg_status ensure_task_scratch(hfg_ctx *c) {
   const size_t nq = c->qclasses.size();
@@ -1372,12 +1376,14 @@ static hfg_status ensure_task_scratch(hfg_ctx *c) {
       total += std::max(c->qclasses[i].tasks.size(), c->qclasses[i].gtasks.size());
     }
     HFG_CUDA(cudaMalloc((void **)&c->d_task_active, std::max<size_t>(1, total) * sizeof(Task)));
-    HFG_CUDA(cudaMalloc((void **)&c->d_task_counts, std::max<size_t>(1, nq) * sizeof(int)));
   }
-  if (!c->d_queue) HFG_CUDA(cudaMalloc((void **)&c->d_queue, std::max<size_t>(1, nq) * sizeof(int)));
-  return HFG_OK;
+  if (!c->d_task_counts) HFG_CUDA(cudaMalloc((void **)&c->d_task_counts, std::max<size_t>(1, nq) * sizeof(int)));
+  return ensure_queue(c);
 }
 
+// Tasks of active molecules, in the class's order up to warp-sized groups:
+// each warp writes its kept tasks as one contiguous run (ballot + one
+// atomic per warp).
 __global__ void compact_active_tasks(const Task *__restrict__ tasks, int ntasks, const int *__restrict__ bra_list,
                                      const int *__restrict__ pair_mol, const unsigned char *__restrict__ active,
                                      Task *__restrict__ out, int *count) {

@@ -192,9 +192,25 @@ def precision_contexts_hold_no_grouped_lists(L):
     assert n > 10
 
 
+def plain_builds_hold_no_compaction_lists(L):
+    """A plain grouped build allocates its work-queue counters, not a copy of
+    the task lists."""
+    os.environ["HFG_GROUP_MIN_TASKS"] = "0"
+    eng = E.Engine(*molecules.water_cluster(4, seed=1), "6-31g*")
+    eng.set_profiling(True)
+    tasks = sum(c["tasks"] for c in eng.class_profile())
+    for k in ("(21|11)", "(21|20)", "(21|21)", "(22|10)", "(22|11)", "(22|20)", "(22|21)"):
+        eng.set_class_path(k, True)  # no scratch
+    start = L.fake_live_bytes()
+    eng.fock_rhf(np.eye(eng.nbf))
+    matrices = 4 * 8 * eng.nbf ** 2  # P, G, J, K
+    assert L.fake_live_bytes() - start < matrices + 4096 < matrices + 16 * tasks
+    _sound(L)
+
+
 CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back,
                               contexts_on_two_devices, grouped_runs,
-                              precision_contexts_hold_no_grouped_lists)]
+                              precision_contexts_hold_no_grouped_lists, plain_builds_hold_no_compaction_lists)]
 
 
 @pytest.mark.parametrize("case", CASES)
