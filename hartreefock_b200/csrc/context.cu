@@ -829,8 +829,9 @@ static int grid_for(const hfg_ctx *c, int ntasks, int cls) {
   return std::max(1, std::min(blocks, c->num_sms * bps));
 }
 
-// Grouped launch: one warp per task, taken from the device queue, one block of
-// as many warps as the registers hold per SM.  Smaller blocks measured slower
+// Grouped launch: one warp per task, taken from the device queue where the
+// launch has one (direct and asynchronous batched builds), grid-stride
+// otherwise; one block of as many warps as the registers hold per SM.  Smaller blocks measured slower
 // also beside other classes: (H2O)32 / 6-31G* build on concurrent streams
 // 22.2 ms, with blocks of 8 warps 25.0 (one per SM) and 23.5 (two), of 4 warps
 // 26.9; (H2O)16 4.88 against 5.40, 5.19 and 5.75.
@@ -2338,7 +2339,7 @@ hfg_status hfg_autotune(hfg_ctx *c, const double *dP, int32_t *chosen, int32_t c
   }
   for (auto &q : c->qclasses) {
     if (kSplit[q.cls] || kWarp[q.cls] || q.tasks.empty()) continue;
-    ClassLaunch cl = base_launch(c, q, true, !c->precision_form() && uses_group(c, q));
+    ClassLaunch cl = base_launch(c, q, true);  // the cap is the one-bra kernel's (grid_for)
     if (cl.ntasks == 0) continue;
     cl.Da = dP;
     cl.Dt = dP;
@@ -2462,11 +2463,17 @@ hfg_status hfg_autotune_tasks(hfg_ctx *c, const double *dP, int32_t *chosen, int
       cl.Dt = dP;
       cl.J = c->d_J;
       cl.Ka = c->d_Ka;
+      // grouped launches take their tasks from the queue, as builds do
+      if (cl.masks) {
+        if ((st = ensure_queue(c)) != HFG_OK) return st;
+        cl.queue = c->d_queue + (&q - c->qclasses.data());
+      }
       int launches = 0;
-      if ((st = launch_class(c, q, cl, kJkRhf, ref, 0, s, &launches)) != HFG_OK) return st;
-      HFG_CUDA(cudaEventRecord(c->ev0, s));
-      for (int r = 0; r < 2; ++r)
+      for (int r = 0; r < 3; ++r) {
+        if (r == 1) HFG_CUDA(cudaEventRecord(c->ev0, s));
+        if (cl.queue) HFG_CUDA(cudaMemsetAsync(cl.queue, 0, sizeof(int), s));
         if ((st = launch_class(c, q, cl, kJkRhf, ref, 0, s, &launches)) != HFG_OK) return st;
+      }
       HFG_CUDA(cudaEventRecord(c->ev1, s));
       HFG_CUDA(cudaEventSynchronize(c->ev1));
       HFG_CUDA(cudaGetLastError());

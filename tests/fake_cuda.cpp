@@ -318,7 +318,7 @@ cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **args, size_t smem
   if (has("eri_group_kernel") || has("eri_class_kernel") || has("eri_warp_kernel") || has("eri_prim_split_kernel") ||
       has("eri_hrr_")) {
     const ClassLaunch &cl = *static_cast<const ClassLaunch *>(args[1]);
-    log_ += name + "\n";
+    log_ += name + (cl.queue ? " queue\n" : "\n");
     use(cl.tasks, sizeof(Task) * (size_t)(cl.task_offset + cl.ntasks), name + " tasks");
     use(cl.bra_list, 4, name + " bra list");
     use(cl.ket_list, 4, name + " ket list");

@@ -208,9 +208,28 @@ def plain_builds_hold_no_compaction_lists(L):
     _sound(L)
 
 
+def autotuners_time_what_they_set(L):
+    """The grid autotuner launches the kernels with a grid cap; the task
+    autotuner the grouped ones as builds do, from the queue."""
+    os.environ["HFG_GROUP_MIN_TASKS"] = "0"
+    eng = E.Engine(*molecules.water_cluster(2, seed=1), "6-31g*")
+    P = (ctypes.c_double * eng.nbf ** 2)()
+    chosen, n = (ctypes.c_int32 * 500)(), ctypes.c_int32()
+    L.fake_clear()
+    E._check(L.hfg_autotune(eng._h, P, chosen, 500, ctypes.byref(n), None))
+    log = L.fake_log().decode()
+    assert n.value > 8 and "eri_class_kernel" in log and "eri_group_kernel" not in log
+    L.fake_clear()
+    E._check(L.hfg_autotune_tasks(eng._h, P, chosen, 500, ctypes.byref(n), None))
+    grouped = [line for line in L.fake_log().decode().splitlines() if "eri_group_kernel" in line]
+    assert grouped and all(line.endswith(" queue") for line in grouped)
+    _sound(L)
+
+
 CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back,
                               contexts_on_two_devices, grouped_runs,
-                              precision_contexts_hold_no_grouped_lists, plain_builds_hold_no_compaction_lists)]
+                              precision_contexts_hold_no_grouped_lists, plain_builds_hold_no_compaction_lists,
+                              autotuners_time_what_they_set)]
 
 
 @pytest.mark.parametrize("case", CASES)
