@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/hfgpu.h"
+#include "device_alloc.h"
 #include "eri_dispatch.cuh"
 #include "eri_group_dispatch.cuh"
 #include "eri_split_dispatch.cuh"
@@ -139,7 +140,7 @@ template <class T>
 static hfg_status upload(T **dst, const std::vector<T> &src) {
   *dst = nullptr;
   if (src.empty()) return HFG_OK;
-  HFG_CUDA(cudaMalloc((void **)dst, src.size() * sizeof(T)));
+  HFG_CUDA(device_alloc(dst, src.size() * sizeof(T)));
   HFG_CUDA(cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
   // a pageable-to-device cudaMemcpy returns once the data is staged; the DMA
   // itself is queued on the legacy default stream, which the context's
@@ -740,7 +741,7 @@ static hfg_status make_group_layout(hfg_ctx *c) {
     tmp.ptrs.push_back(d_records);
     if (st != HFG_OK || (st = upload(&L.d_gpairs, L.gpairs)) != HFG_OK || (st = upload(&L.d_block_off, off)) != HFG_OK)
       return st;
-    HFG_CUDA(cudaMalloc((void **)&L.d_blocks, (size_t)total * kKetStride * sizeof(double)));
+    HFG_CUDA(device_alloc(&L.d_blocks, (size_t)total * kKetStride * sizeof(double)));
     const int nb = (int)off.size();
     fill_ket_blocks<<<std::max(1, std::min(c->num_sms * 8, (nb + 7) / 8)), 256, 0, c->stream>>>(
         c->view(), L.d_pairs, (int)L.pairs.size(), L.d_block_off, d_records, nb, L.d_blocks);
@@ -776,7 +777,7 @@ static hfg_status upload_groups(hfg_ctx *c) {
   for (auto &q : c->qclasses) {
     if (q.gtasks.empty()) continue;
     if (const hfg_status st = upload(&q.d_gtasks, q.gtasks); st != HFG_OK) return st;
-    HFG_CUDA(cudaMalloc((void **)&q.d_gmasks, q.ngmasks * sizeof(uint2)));
+    HFG_CUDA(device_alloc(&q.d_gmasks, q.ngmasks * sizeof(uint2)));
     const ClassEntry &e = kClasses[q.cls];
     const int grid = std::max(1, std::min(c->num_sms * 8, ((int)q.gtasks.size() + 7) / 8));
     group_masks_kernel<<<grid, 256, 0, c->stream>>>(c->view(), c->pclass[q.bra_pc].d_gpairs, c->pclass[q.ket_pc].d_pairs,
@@ -985,7 +986,7 @@ __global__ void finalize_uhf_incremental(const double *J, const double *Ka, cons
 
 static hfg_status ensure(double **p, size_t count) {
   if (*p) return HFG_OK;
-  HFG_CUDA(cudaMalloc((void **)p, count * sizeof(double)));
+  HFG_CUDA(device_alloc(p, count * sizeof(double)));
   return HFG_OK;
 }
 
@@ -1092,7 +1093,7 @@ static hfg_status grow_scratch(hfg_ctx *c, int slot, size_t need) {
   cudaFree(c->d_scratch[slot]);
   c->d_scratch[slot] = nullptr;
   c->scratch_doubles[slot] = 0;
-  HFG_CUDA(cudaMalloc((void **)&c->d_scratch[slot], need * sizeof(double)));
+  HFG_CUDA(device_alloc(&c->d_scratch[slot], need * sizeof(double)));
   c->scratch_doubles[slot] = need;
   ++c->config_version;  // a captured graph holds the old region
   return HFG_OK;
@@ -1160,8 +1161,8 @@ static hfg_status direct_build_body(hfg_ctx *c, bool uhf, const double *dPa, con
   const double *Da = dPa, *Db = dPb;
   if (precise) {
     const int ns = c->nshells;
-    if (!c->d_shell_dmax) HFG_CUDA(cudaMalloc((void **)&c->d_shell_dmax, (size_t)ns * ns * sizeof(float)));
-    if (!c->d_counters) HFG_CUDA(cudaMalloc((void **)&c->d_counters, 2 * sizeof(unsigned long long)));
+    if (!c->d_shell_dmax) HFG_CUDA(device_alloc(&c->d_shell_dmax, (size_t)ns * ns * sizeof(float)));
+    if (!c->d_counters) HFG_CUDA(device_alloc(&c->d_counters, 2 * sizeof(unsigned long long)));
     HFG_CUDA(cudaMemsetAsync(c->d_counters, 0, 2 * sizeof(unsigned long long), s));
     if (incremental) {
       for (int k = 0; k < (uhf ? 2 : 1); ++k)
@@ -1360,7 +1361,7 @@ __global__ void finalize_uhf_batch(const double *J, const double *Ka, const doub
 
 // Work-queue counters, one per quartet class.
 static hfg_status ensure_queue(hfg_ctx *c) {
-  if (!c->d_queue) HFG_CUDA(cudaMalloc((void **)&c->d_queue, std::max<size_t>(1, c->qclasses.size()) * sizeof(int)));
+  if (!c->d_queue) HFG_CUDA(device_alloc(&c->d_queue, std::max<size_t>(1, c->qclasses.size()) * sizeof(int)));
   return HFG_OK;
 }
 
@@ -1376,9 +1377,9 @@ static hfg_status ensure_task_scratch(hfg_ctx *c) {
       c->task_base[i] = (int)total;
       total += std::max(c->qclasses[i].tasks.size(), c->qclasses[i].gtasks.size());
     }
-    HFG_CUDA(cudaMalloc((void **)&c->d_task_active, std::max<size_t>(1, total) * sizeof(Task)));
+    HFG_CUDA(device_alloc(&c->d_task_active, std::max<size_t>(1, total) * sizeof(Task)));
   }
-  if (!c->d_task_counts) HFG_CUDA(cudaMalloc((void **)&c->d_task_counts, std::max<size_t>(1, nq) * sizeof(int)));
+  if (!c->d_task_counts) HFG_CUDA(device_alloc(&c->d_task_counts, std::max<size_t>(1, nq) * sizeof(int)));
   return ensure_queue(c);
 }
 
@@ -1875,7 +1876,7 @@ static hfg_status create_context(const hfg_shells *sh, const int *shell_mol, int
       (st = upload(&ctx->d_pair_ao_b, paob)) != HFG_OK || (st = upload(&ctx->d_pair_AB, pab)) != HFG_OK ||
       (st = upload(&ctx->d_boys, boys_table_host())) != HFG_OK)
     return st;
-  HFG_CUDA(cudaMalloc((void **)&ctx->d_pair_Q, (size_t)np * sizeof(double)));
+  HFG_CUDA(device_alloc(&ctx->d_pair_Q, (size_t)np * sizeof(double)));
   HFG_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   HFG_CUDA(cudaEventCreate(&ctx->ev0));
   HFG_CUDA(cudaEventCreate(&ctx->ev1));
@@ -2022,7 +2023,7 @@ hfg_status hfg_eri_packed(hfg_ctx *c, double *host_out, int64_t count) {
   if (count != hfg_packed_size(c->nbf)) return fail(HFG_INVALID_ARG, "count != hfg_packed_size(nbf)");
   HFG_CUDA(cudaSetDevice(c->device));
   double *d = nullptr;
-  HFG_CUDA(cudaMalloc((void **)&d, (size_t)count * sizeof(double)));
+  HFG_CUDA(device_alloc(&d, (size_t)count * sizeof(double)));
   hfg_status st = stored_build(c, d, count, c->stream);
   if (st == HFG_OK) st = finish_timing(c);
   if (st == HFG_OK) {

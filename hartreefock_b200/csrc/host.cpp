@@ -21,6 +21,7 @@
 #include <thread>
 
 #include "../../include/hfgpu_driver.h"
+#include "device_alloc.h"
 #include "../../include/hfgpu_host.hpp"
 #include "driver_internal.h"
 #include "scf_device.h"
@@ -87,7 +88,7 @@ void grow(double **p, size_t *cap, size_t need) {
   if (need <= *cap) return;
   cudaFree(*p);
   *p = nullptr;
-  if (cudaMalloc(p, need * sizeof(double)) != cudaSuccess) throw std::runtime_error("cudaMalloc (gemm)");
+  if (hfg::device_alloc(p, need * sizeof(double)) != cudaSuccess) throw std::runtime_error("cudaMalloc (gemm)");
   *cap = need;
 }
 }  // namespace
@@ -195,13 +196,13 @@ void eigh(const Matrix &a, std::vector<double> &w, Matrix &v) {
     cudaFree(s.dW);
     cudaFree(s.work);
     cudaFree(s.info);
-    check_cuda(cudaMalloc(&s.dA, sizeof(double) * n * n), "cudaMalloc");
-    check_cuda(cudaMalloc(&s.dW, sizeof(double) * n), "cudaMalloc");
-    check_cuda(cudaMalloc(&s.info, sizeof(int)), "cudaMalloc");
+    check_cuda(hfg::device_alloc(&s.dA, sizeof(double) * n * n), "cudaMalloc");
+    check_cuda(hfg::device_alloc(&s.dW, sizeof(double) * n), "cudaMalloc");
+    check_cuda(hfg::device_alloc(&s.info, sizeof(int)), "cudaMalloc");
     check_solver(cusolverDnDsyevd_bufferSize(s.h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, s.dA, n, s.dW,
                                              &s.lwork),
                  "dsyevd_bufferSize");
-    check_cuda(cudaMalloc(&s.work, sizeof(double) * s.lwork), "cudaMalloc");
+    check_cuda(hfg::device_alloc(&s.work, sizeof(double) * s.lwork), "cudaMalloc");
     s.cap = n;
   }
   // symmetric input: row-major == column-major
@@ -482,7 +483,7 @@ double MolecularOrbitalsIntegralsRepository::getElectronElectron(unsigned p, uns
     if (C.rows() != n_ || C.cols() != n_) throw std::invalid_argument("MO coefficients: nbf x nbf expected");
     const size_t nn = (size_t)n_ * n_;
     double *dC = nullptr, *dX = nullptr;
-    if (cudaMalloc(&dC, nn * sizeof(double)) != cudaSuccess || cudaMalloc(&dX, nn * nn * sizeof(double)) != cudaSuccess) {
+    if (hfg::device_alloc(&dC, nn * sizeof(double)) != cudaSuccess || hfg::device_alloc(&dX, nn * nn * sizeof(double)) != cudaSuccess) {
       cudaFree(dC);
       throw std::runtime_error("MolecularOrbitalsIntegralsRepository: device allocation");
     }

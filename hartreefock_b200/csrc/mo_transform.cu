@@ -16,17 +16,19 @@
 // 2 N^4 nj + 2 N^3 nj nb + ... operations, where a product with the pair
 // coefficients C_j C_b takes 2 N^4 nj nb: (H2O)4 / 6-31G* (N = 76, 20 x 56) 9.3 ->
 // 3.7 ms, and 1.6 ms with the handle and the workspace kept (MoState), 1.1 ms of
-// it the stored build.  FP64 throughout; cuBLAS for the plain GEMMs.  The unpacking kernel is bound by the packed table's gathers.  Memory:
-// N^4 + N^4/8 doubles for the tables, at most 2 N^2 max(N max(nj, ni), ov) for
-// the intermediates.
+// it the stored build.  FP64 throughout; cuBLAS for the plain GEMMs.  The
+// unpacking kernel is bound by the packed table's gathers.  Memory: N^4 + N^4/8
+// doubles for the tables, 3 N^2 ov for the intermediates (T, in slabs of m, and Y).
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <string>
+#include <mutex>
 #include <vector>
 
 #include "../../include/hfgpu.h"
+#include "device_alloc.h"
 
 namespace hfg {
 hfg_status fail_external(hfg_status st, const std::string &msg);
@@ -108,25 +110,70 @@ struct Buffers {
     for (void *p : ptrs) cudaFree(p);
   }
   cudaError_t get(double **p, size_t count) {
-    cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(double));
+    cudaError_t e = hfg::device_alloc(p, count * sizeof(double));
     if (e == cudaSuccess) ptrs.push_back(*p);
     return e;
   }
 };
 
 // What a context keeps between its transforms: the cuBLAS handle, and the
-// workspace of the last one while it is at most kMoKeepBytes (allocating and
-// freeing 400 MB took from 1 to 30 ms of a call).  Both go with the context.
+// workspace of the last one (allocating and freeing 400 MB took from 1 to 30 ms
+// of a call).  The workspaces that idle contexts keep on a device come to at
+// most kMoKeepBytes together, the longest unused going first; all of them are
+// given back when an allocation of the library finds no memory, and a context's
+// goes with it.
 constexpr size_t kMoKeepBytes = size_t(1) << 30;
 struct MoState {
   cublasHandle_t blas = nullptr;
   double *work = nullptr;
   size_t count = 0;
-  ~MoState() {
-    cudaFree(work);
-    if (blas) cublasDestroy(blas);
-  }
+  int device = 0;
+  bool busy = false;
+  MoState();
+  ~MoState();
 };
+std::mutex &kept_mutex() {
+  static std::mutex *m = new std::mutex;  // contexts may go after static objects do
+  return *m;
+}
+std::vector<MoState *> &kept() {  // every context's state, the longest unused first
+  static auto *v = new std::vector<MoState *>;
+  return *v;
+}
+MoState::MoState() {
+  cudaGetDevice(&device);
+  std::lock_guard<std::mutex> lock(kept_mutex());
+  kept().push_back(this);
+}
+MoState::~MoState() {
+  {
+    std::lock_guard<std::mutex> lock(kept_mutex());
+    kept().erase(std::find(kept().begin(), kept().end(), this));
+  }
+  cudaFree(work);
+  if (blas) cublasDestroy(blas);
+}
+// Frees idle workspaces on the current device until at most `most` bytes of
+// them are left; whether any went.
+bool give_back(size_t most) {
+  int device = 0;
+  cudaGetDevice(&device);
+  std::lock_guard<std::mutex> lock(kept_mutex());
+  const auto idle = [&](const MoState *s) { return s->device == device && !s->busy && s->work; };
+  size_t bytes = 0;
+  for (const MoState *s : kept()) bytes += idle(s) ? s->count * sizeof(double) : 0;
+  bool any = false;
+  for (MoState *s : kept()) {
+    if (bytes <= most) break;
+    if (!idle(s)) continue;
+    bytes -= s->count * sizeof(double);
+    cudaFree(s->work);
+    s->work = nullptr;
+    s->count = 0;
+    any = true;
+  }
+  return any;
+}
 MoState *context_state(hfg_ctx *ctx) {
   MoState *st = static_cast<MoState *>(hfg::ctx_handle(ctx));
   if (!st) {
@@ -142,12 +189,32 @@ MoState *context_state(hfg_ctx *ctx) {
 
 // The unpacked AO table M[(m n),(l s)] of the context (stored-mode build) and
 // the intermediates of the blocks that follow, of at most `ov_max` index pairs
-// on either side.
+// on either side.  Holds the context's workspace while it lives.
 struct MoTables {
   int n = 0;
   double *M = nullptr, *T = nullptr, *Y = nullptr;  // T: 2 N^2 ov_max, Y: N^2 ov_max
   long long cap = 0;
   cublasHandle_t blas = nullptr;
+  MoState *state = nullptr;
+  bool finished = false;  // nothing queued uses the tables any more
+  MoTables() = default;
+  MoTables(const MoTables &) = delete;
+  void hold(MoState *s) {
+    std::lock_guard<std::mutex> lock(kept_mutex());
+    state = s;
+    state->busy = true;
+  }
+  ~MoTables() {
+    if (!state) return;
+    if (!finished) cudaDeviceSynchronize();
+    {
+      std::lock_guard<std::mutex> lock(kept_mutex());
+      state->busy = false;
+      kept().erase(std::find(kept().begin(), kept().end(), state));
+      kept().push_back(state);
+    }
+    give_back(kMoKeepBytes);
+  }
 };
 
 hfg_status prepare(hfg_ctx *ctx, long long ov_max, cudaStream_t s, Buffers &buf, MoTables &t, const char *who) {
@@ -159,6 +226,7 @@ hfg_status prepare(hfg_ctx *ctx, long long ov_max, cudaStream_t s, Buffers &buf,
   if (!state || cublasSetStream(state->blas, s) != CUBLAS_STATUS_SUCCESS)
     return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": cuBLAS handle");
   t.blas = state->blas;
+  t.hold(state);
   const size_t words = (size_t)(nn * nn + 3 * nn * ov_max + count);  // M, T, Y, packed
   double *all = state->work;
   if (state->count < words) {
@@ -166,13 +234,14 @@ hfg_status prepare(hfg_ctx *ctx, long long ov_max, cudaStream_t s, Buffers &buf,
     state->work = nullptr;
     state->count = 0;
     size_t freeb = 0, totalb = 0;
-    cudaMemGetInfo(&freeb, &totalb);
     const double need = 8.0 * (double)words;
+    cudaMemGetInfo(&freeb, &totalb);
+    if (need > 0.9 * (double)freeb && give_back(0)) cudaMemGetInfo(&freeb, &totalb);
     if (need > 0.9 * (double)freeb)
       return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": the unpacked AO table does not fit (" +
                                                     std::to_string(need / 1e9) + " GB needed)");
     const bool keep = words * sizeof(double) <= kMoKeepBytes;
-    const cudaError_t e = keep ? cudaMalloc(reinterpret_cast<void **>(&all), words * sizeof(double)) : buf.get(&all, words);
+    const cudaError_t e = keep ? hfg::device_alloc(&all, words * sizeof(double)) : buf.get(&all, words);
     if (e != cudaSuccess) return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": " + cudaGetErrorString(e));
     if (keep) {
       state->work = all;
@@ -234,8 +303,9 @@ hfg_status block(MoTables &t, Range i, Range a, Range j, Range b, double *dX, cu
   return HFG_OK;
 }
 
-hfg_status finish(cudaStream_t s, const char *who) {
+hfg_status finish(MoTables &t, cudaStream_t s, const char *who) {
   cudaError_t e = cudaStreamSynchronize(s);
+  t.finished = e == cudaSuccess;
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": " + cudaGetErrorString(e));
   return HFG_OK;
@@ -252,10 +322,19 @@ hfg_status transform(hfg_ctx *ctx, const double *dC, int i0, int ni, int a0, int
   if (st != HFG_OK) return st;
   st = block(t, {dC, i0, ni}, {dC, a0, na}, {dC, i0, ni}, {dC, a0, na}, dX, s, "hfg_mo_eri_ovov");
   if (st != HFG_OK) return st;
-  return finish(s, "hfg_mo_eri_ovov");
+  return finish(t, s, "hfg_mo_eri_ovov");
 }
 
 }  // namespace
+
+cudaError_t hfg::device_alloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && give_back(0)) {
+    cudaGetLastError();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
 
 extern "C" hfg_status hfg_mo_eri_ovov(hfg_ctx *ctx, const double *dC, int32_t i0, int32_t ni, int32_t a0, int32_t na,
                                       double *dX, void *stream) {
@@ -372,7 +451,7 @@ extern "C" hfg_status hfg_mp2_uhf(hfg_ctx *ctx, const double *Cp, const double *
                                                       eps + q.i.first, eps + q.a.first, eps + q.j.first,
                                                       eps + q.b.first, dOut);
   }
-  if ((st = finish(s, who)) != HFG_OK) return st;
+  if ((st = finish(t, s, who)) != HFG_OK) return st;
   double sum = 0;
   e = cudaMemcpy(&sum, dOut, sizeof(double), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": " + cudaGetErrorString(e));
@@ -413,7 +492,7 @@ extern "C" hfg_status hfg_mo_eri_full(hfg_ctx *ctx, const double *dC, double *dX
   hfg_status st = prepare(ctx, (long long)n * n, s, buf, t, who);
   if (st != HFG_OK) return st;
   if ((st = block(t, {dC, 0, n}, {dC, 0, n}, {dC, 0, n}, {dC, 0, n}, dX, s, who)) != HFG_OK) return st;
-  return finish(s, who);
+  return finish(t, s, who);
 }
 
 // SpinOrbitalsElectronElectronIntegralsRepository::Compute

@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "../../include/hfgpu.h"
+#include "device_alloc.h"
 #include "eri_kernels.cuh"
 
 namespace hfg {
@@ -265,7 +266,7 @@ struct DeviceArray {
     if (p) cudaFree(p);
   }
   cudaError_t upload(const std::vector<T> &v) {
-    cudaError_t e = cudaMalloc(&p, std::max<size_t>(1, v.size()) * sizeof(T));
+    cudaError_t e = hfg::device_alloc(&p, std::max<size_t>(1, v.size()) * sizeof(T));
     if (e != cudaSuccess || v.empty()) return e;
     e = cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
     // the staged copy's DMA runs on the legacy stream; the kernels below run
@@ -362,7 +363,7 @@ hfg_status one_electron_all(const hfg_shells *sh, const double *nuc_xyz, const i
   if (e == cudaSuccess) e = d_nuc.upload(nuc);
   if (e == cudaSuccess) e = d_boys.upload(boys_table_for_external());
   const size_t nn = (size_t)n * n;
-  if (e == cudaSuccess) e = cudaMalloc(&d_out.p, 6 * nn * sizeof(double));
+  if (e == cudaSuccess) e = hfg::device_alloc(&d_out.p, 6 * nn * sizeof(double));
   if (e == cudaSuccess) e = cudaMemsetAsync(d_out.p, 0, 6 * nn * sizeof(double), os.s);
   if (e != cudaSuccess) return fail_external(HFG_OOM_BUDGET, std::string("hfg_one_electron: ") + cudaGetErrorString(e));
   double *dS = d_out.p, *dT = dS + nn, *dV = dT + nn, *dMx = dV + nn, *dMy = dMx + nn, *dMz = dMy + nn;

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/hfgpu.h"
+#include "device_alloc.h"
 #include "scf_device.h"
 
 namespace hfgpu {
@@ -72,23 +73,23 @@ DeviceScf::DeviceScf(int n, int device) : n_(n), device_(device) {
   ck(cusolverDnSetStream(solver_, stream_), "cusolverDnSetStream");
   const size_t nn = (size_t)n * n;
   for (double **p : {&h_, &S_, &V_, &T1_, &T2_, &Ft_, &W_, &err_})
-    ck(cudaMalloc((void **)p, nn * sizeof(double)), "cudaMalloc");
+    ck(hfg::device_alloc(p, nn * sizeof(double)), "cudaMalloc");
   for (int s = 0; s < 2; ++s)
-    for (double **p : {&P_[s], &Pn_[s], &F_[s], &G_[s], &C_[s]}) ck(cudaMalloc((void **)p, nn * sizeof(double)), "cudaMalloc");
-  ck(cudaMalloc((void **)&w_, 2 * (size_t)n * sizeof(double)), "cudaMalloc");
-  ck(cudaMalloc((void **)&info_, sizeof(int)), "cudaMalloc");
-  ck(cudaMalloc((void **)&occ_dev_, (size_t)n * sizeof(int)), "cudaMalloc");
-  ck(cudaMalloc((void **)&scalars_, 64 * sizeof(double)), "cudaMalloc");
-  ck(cudaMalloc((void **)&coef_, 16 * sizeof(double)), "cudaMalloc");
+    for (double **p : {&P_[s], &Pn_[s], &F_[s], &G_[s], &C_[s]}) ck(hfg::device_alloc(p, nn * sizeof(double)), "cudaMalloc");
+  ck(hfg::device_alloc(&w_, 2 * (size_t)n * sizeof(double)), "cudaMalloc");
+  ck(hfg::device_alloc(&info_, sizeof(int)), "cudaMalloc");
+  ck(hfg::device_alloc(&occ_dev_, (size_t)n * sizeof(int)), "cudaMalloc");
+  ck(hfg::device_alloc(&scalars_, 64 * sizeof(double)), "cudaMalloc");
+  ck(hfg::device_alloc(&coef_, 16 * sizeof(double)), "cudaMalloc");
   ck(cudaMallocHost((void **)&host_scalars_, 64 * sizeof(double)), "cudaMallocHost");
   ck(cudaMallocHost((void **)&host_info_, sizeof(int)), "cudaMallocHost");
   ck(cudaMallocHost((void **)&host_w_, 2 * (size_t)n * sizeof(double)), "cudaMallocHost");
   ck(cusolverDnDsyevd_bufferSize(solver_, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, Ft_, n, w_, &lwork_),
      "dsyevd_bufferSize");
-  ck(cudaMalloc((void **)&work_, (size_t)std::max(lwork_, 1) * sizeof(double)), "cudaMalloc");
+  ck(hfg::device_alloc(&work_, (size_t)std::max(lwork_, 1) * sizeof(double)), "cudaMalloc");
   for (int s = 0; s < 2; ++s) {
-    ck(cudaMalloc((void **)&diis_F_[s], kDiisKeep * nn * sizeof(double)), "cudaMalloc");
-    ck(cudaMalloc((void **)&diis_E_[s], kDiisKeep * nn * sizeof(double)), "cudaMalloc");
+    ck(hfg::device_alloc(&diis_F_[s], kDiisKeep * nn * sizeof(double)), "cudaMalloc");
+    ck(hfg::device_alloc(&diis_E_[s], kDiisKeep * nn * sizeof(double)), "cudaMalloc");
   }
   for (auto &e : ev_) ck(cudaEventCreate(&e), "cudaEventCreate");
 }
@@ -360,14 +361,14 @@ extern "C" hfg_status hfg_eigh_batched(const double *dA, double *dV, double *dW,
         ck(cudaStreamSynchronize(s), "sync");
         if (e.dwork) cudaFree(e.dwork);
         e.dwork = nullptr;
-        ck(cudaMalloc(&e.dwork, need), "cudaMalloc eigh workspace");
+        ck(hfg::device_alloc(&e.dwork, need), "cudaMalloc eigh workspace");
         e.dbytes = need;
       }
       if (batch > e.info_cap) {
         ck(cudaStreamSynchronize(s), "sync");
         if (e.info) cudaFree(e.info);
         e.info = nullptr;
-        ck(cudaMalloc(&e.info, sizeof(int) * batch), "cudaMalloc eigh info");
+        ck(hfg::device_alloc(&e.info, sizeof(int) * batch), "cudaMalloc eigh info");
         e.info_cap = batch;
       }
       const size_t nn = (size_t)n * n;
@@ -385,7 +386,7 @@ extern "C" hfg_status hfg_eigh_batched(const double *dA, double *dV, double *dW,
       ck(cudaStreamSynchronize(s), "sync");
       if (e.dwork) cudaFree(e.dwork);
       e.dwork = nullptr;
-      ck(cudaMalloc(&e.dwork, dneed), "cudaMalloc eigh workspace");
+      ck(hfg::device_alloc(&e.dwork, dneed), "cudaMalloc eigh workspace");
       e.dbytes = dneed;
     }
     if (hneed > e.hwork.size()) e.hwork.resize(hneed);
@@ -393,7 +394,7 @@ extern "C" hfg_status hfg_eigh_batched(const double *dA, double *dV, double *dW,
       ck(cudaStreamSynchronize(s), "sync");
       if (e.info) cudaFree(e.info);
       e.info = nullptr;
-      ck(cudaMalloc(&e.info, sizeof(int) * batch), "cudaMalloc eigh info");
+      ck(hfg::device_alloc(&e.info, sizeof(int) * batch), "cudaMalloc eigh info");
       e.info_cap = batch;
     }
     ck(cusolverDnXsyevBatched(e.handle, e.params, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, CUDA_R_64F, dV,

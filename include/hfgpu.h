@@ -243,15 +243,17 @@ hfg_status hfg_moments(const hfg_shells *shells, int32_t device, double *Mx, dou
  * reference's C).  Replaces MolecularOrbitalsIntegralsRepository::
  * getElectronElectron (IntegralsRepository.h:190-291) for that block.  Uses
  * the context's stored-mode table (its screening and ERI convention),
- * unpacked on the device: needs about 9/8 nbf^4 doubles free, else
- * HFG_OOM_BUDGET.  Single-molecule contexts only. */
+ * unpacked on the device: needs 9/8 nbf^4 + 3 nbf^2 ni na doubles free, else
+ * HFG_OOM_BUDGET.  The context keeps that workspace for its next transform:
+ * idle contexts at most 1 GiB of it together per device, which goes with the
+ * context, or when an allocation of this library finds no memory.
+ * Single-molecule contexts only. */
 hfg_status hfg_mo_eri_ovov(hfg_ctx *ctx, const double *dC, int32_t i0, int32_t ni, int32_t a0, int32_t na, double *dX,
                            void *stream);
 /* The whole MO tensor (pq|rs) for every orbital of dC (device, row-major
  * nbf x nbf), as dX[(p q),(r s)] (nbf^2 x nbf^2, row-major): the elements
  * MolecularOrbitalsIntegralsRepository::getElectronElectron(p, q, r, s, C)
- * returns (IntegralsRepository.h:190-291).  Needs about 11/8 nbf^4 doubles
- * free.  Single-molecule contexts only. */
+ * returns (IntegralsRepository.h:190-291).  Needs 33/8 nbf^4 doubles free.  Single-molecule contexts only. */
 hfg_status hfg_mo_eri_full(hfg_ctx *ctx, const double *dC, double *dX, void *stream);
 /* SpinOrbitalsElectronElectronIntegralsRepository::Compute
  * (SpinOrbitalsElectronElectronIntegralsRepository.cpp:30-52) for host C

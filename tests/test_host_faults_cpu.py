@@ -226,10 +226,46 @@ def autotuners_time_what_they_set(L):
     _sound(L)
 
 
+def transform_workspaces_are_given_back(L):
+    """Workspaces that idle contexts keep: bounded together, given back to an
+    allocation that finds no memory, and gone with their context."""
+    Z, xyz = molecules.water_cluster(4, seed=1)
+    eps = np.arange(76, dtype=float)
+    start = L.fake_live_bytes()
+    engines = [E.Engine(Z, xyz, "6-31g*") for _ in range(4)]
+    for e in engines:
+        e.fock_rhf(np.eye(76))
+    none = L.fake_live_bytes()
+    for e in engines + engines[:2]:  # 450 MB each
+        e.mp2_rhf(np.eye(76), eps, 20)
+        assert L.fake_live_bytes() - none <= (1 << 30) + (64 << 20)
+    kept = L.fake_live_bytes() - none
+    assert kept > 256 << 20  # and kept they are
+    L.fake_fail_allocation(1)
+    other = E.Engine(Z, xyz, "6-31g*")  # finds no memory at first
+    assert L.fake_live_bytes() - none < 64 << 20
+    for e in engines:
+        e.mp2_rhf(np.eye(76), eps, 20)
+    for n in (1, 2, 3, 4, 5, 6):  # a transform that fails leaves its context usable
+        for e in engines:
+            L.fake_fail_allocation(n)
+            try:
+                e.mp2_rhf(np.eye(76), eps, 20)
+            except E.HfgError:
+                pass
+            L.fake_fail_allocation(0)
+            e.mp2_rhf(np.eye(76), eps, 20)
+    other.close()
+    for e in engines:
+        e.close()
+    assert L.fake_live_bytes() == start
+    _sound(L)
+
+
 CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back,
                               contexts_on_two_devices, grouped_runs,
                               precision_contexts_hold_no_grouped_lists, plain_builds_hold_no_compaction_lists,
-                              autotuners_time_what_they_set)]
+                              autotuners_time_what_they_set, transform_workspaces_are_given_back)]
 
 
 @pytest.mark.parametrize("case", CASES)
