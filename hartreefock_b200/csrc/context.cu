@@ -15,6 +15,7 @@
 
 #include "../../include/hfgpu.h"
 #include "device_alloc.h"
+#include "driver_internal.h"
 #include "eri_dispatch.cuh"
 #include "eri_group_dispatch.cuh"
 #include "eri_split_dispatch.cuh"
@@ -149,6 +150,9 @@ static hfg_status upload(T **dst, const std::vector<T> &src) {
   HFG_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   return HFG_OK;
 }
+
+static_assert(hfgpu::kPrimPairBytes == sizeof(PrimPair) + sizeof(PrimPairF) + kKetFields * sizeof(double),
+              "the admission estimate's primitive pair");
 
 // Device buffers freed at the end of a scope.
 struct Scoped {

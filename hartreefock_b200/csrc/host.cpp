@@ -1246,7 +1246,7 @@ int64_t job_footprint_bytes(const char *basis_path, int32_t natoms, const int32_
     for (int64_t b = 0; b <= a; ++b) prim_pairs += (int64_t)t.nprim[a] * t.nprim[b];
   const int64_t tasks = pairs * (pairs + 1) / 2 / 32 + pairs;
   const int64_t nn = (int64_t)t.nbf * t.nbf;
-  return 16 * tasks + 144 * prim_pairs + 8 * nn * 32 * (unrestricted ? 2 : 1) + (int64_t(16) << 20);
+  return 16 * tasks + kPrimPairBytes * prim_pairs + 8 * nn * 32 * (unrestricted ? 2 : 1) + (int64_t(16) << 20);
 }
 
 void release_driver_thread() { hfd_release_thread(); }

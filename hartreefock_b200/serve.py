@@ -47,12 +47,17 @@ from .basis_io import basis_path, shell_table
 HFG_OOM_BUDGET = 3
 SERVE_BASES = ("6-31g", "6-31g*", "6-31+g**")
 
+PRIM_PAIR_BYTES = 256  # FP64 record, FP32 record, blocked copy
+
 
 def footprint_bytes(Z, xyz, basis: str, unrestricted: bool = False) -> int:
     """Estimated device bytes of one job, the estimate the native pool uses
     too (job_footprint_bytes in hartreefock_b200/csrc/host.cpp): quartet task
     lists (16 B per task of up to 32 ket pairs over the triangle of shell
-    pairs), primitive-pair tables (96 B FP64 + 48 B FP32 per primitive pair),
+    pairs, before screening: where molecules are large enough for the second
+    list and the masks of the grouped kernels, or the precision form's copy of
+    the list, the screened lists with those are below it), primitive-pair
+    tables (128 B FP64 + 48 B FP32 + 80 B blocked copy per primitive pair),
     the SCF's n x n FP64 matrices (h, S, V, F, P, new P, C, G, work, 2 x 6
     DIIS entries, the incremental history; about 32 per spin), plus a fixed
     16 MiB for the Boys table, counters and library handles."""
@@ -62,7 +67,7 @@ def footprint_bytes(Z, xyz, basis: str, unrestricted: bool = False) -> int:
     prim_pairs = int(np.sum(np.triu(np.outer(t.nprim, t.nprim))))
     tasks = pairs * (pairs + 1) // 2 // 32 + pairs
     spins = 2 if unrestricted else 1
-    return int(16 * tasks + 144 * prim_pairs + 8 * t.nbf * t.nbf * 32 * spins + (16 << 20))
+    return int(16 * tasks + PRIM_PAIR_BYTES * prim_pairs + 8 * t.nbf * t.nbf * 32 * spins + (16 << 20))
 
 
 class Job:

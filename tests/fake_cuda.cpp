@@ -121,6 +121,9 @@ int fake_longest_run() {
   return r;
 }
 const char *fake_log() { return log_.c_str(); }
+long long fake_prim_pair_bytes() {
+  return sizeof(hfg::PrimPair) + sizeof(hfg::PrimPairF) + hfg::kKetFields * sizeof(double);
+}
 void fake_clear() {
   bad.clear();
   log_.clear();

@@ -262,10 +262,28 @@ def transform_workspaces_are_given_back(L):
     _sound(L)
 
 
+def admission_counts_the_tables_there_are(L):
+    """The serving estimate's bytes per primitive pair are those of the engine's
+    records, and the estimate covers a context and its first builds."""
+    from hartreefock_b200 import serve
+    L.fake_prim_pair_bytes.restype = ctypes.c_longlong
+    assert serve.PRIM_PAIR_BYTES == L.fake_prim_pair_bytes()
+    for mol, basis in ((molecules.water_cluster(2, seed=1), "6-31g*"), (molecules.alkane(3), "6-31+g**"),
+                       (molecules.water_cluster(8, seed=1), "6-31g*")):
+        start = L.fake_live_bytes()
+        eng = E.Engine(*mol, basis)
+        for k in ("(21|11)", "(21|20)", "(21|21)", "(22|10)", "(22|11)", "(22|20)", "(22|21)"):
+            eng.set_class_path(k, True)
+        eng.fock_rhf(np.eye(eng.nbf))
+        assert L.fake_live_bytes() - start < serve.footprint_bytes(*mol, basis)
+        eng.close()
+
+
 CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back,
                               contexts_on_two_devices, grouped_runs,
                               precision_contexts_hold_no_grouped_lists, plain_builds_hold_no_compaction_lists,
-                              autotuners_time_what_they_set, transform_workspaces_are_given_back)]
+                              autotuners_time_what_they_set, transform_workspaces_are_given_back,
+                              admission_counts_the_tables_there_are)]
 
 
 @pytest.mark.parametrize("case", CASES)
