@@ -5,8 +5,8 @@
 
 namespace hfg {
 
-// cudaMalloc that, where memory is short, first gives back the workspaces that
-// idle contexts keep on the current device (mo_transform.cu) and tries again.
+// cudaMalloc that, where memory is short, first gives back the idle workspaces
+// of the MO transforms on the current device (mo_transform.cu) and tries again.
 cudaError_t device_alloc(void **p, size_t bytes);
 template <class T>
 cudaError_t device_alloc(T **p, size_t bytes) {

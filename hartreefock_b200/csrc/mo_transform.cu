@@ -116,64 +116,92 @@ struct Buffers {
   }
 };
 
-// What a context keeps between its transforms: the cuBLAS handle, and the
-// workspace of the last one (allocating and freeing 400 MB took from 1 to 30 ms
-// of a call).  The workspaces that idle contexts keep on a device come to at
-// most kMoKeepBytes together, the longest unused going first; all of them are
-// given back when an allocation of the library finds no memory, and a context's
-// goes with it.
+// Workspaces between transforms (allocating and freeing 400 MB took from 1 to
+// 30 ms of a call): idle blocks of a device, which the next transform of any of
+// its contexts takes, come to at most kMoKeepBytes, the longest unused going
+// first.  All of them are given back when an allocation of the library finds no
+// memory, and with the last context of the device that ran a transform.
 constexpr size_t kMoKeepBytes = size_t(1) << 30;
-struct MoState {
-  cublasHandle_t blas = nullptr;
-  double *work = nullptr;
-  size_t count = 0;
+struct Workspace {
+  double *p = nullptr;
+  size_t words = 0;
   int device = 0;
-  bool busy = false;
-  MoState();
-  ~MoState();
 };
-std::mutex &kept_mutex() {
-  static std::mutex *m = new std::mutex;  // contexts may go after static objects do
-  return *m;
+struct Pool {
+  std::mutex mutex;
+  std::vector<Workspace> idle;       // the longest unused first
+  std::vector<int> users;            // contexts that ran a transform, by device
+};
+Pool &pool() {
+  static Pool *p = new Pool;  // contexts may go after static objects do
+  return *p;
 }
-std::vector<MoState *> &kept() {  // every context's state, the longest unused first
-  static auto *v = new std::vector<MoState *>;
-  return *v;
-}
-MoState::MoState() {
-  cudaGetDevice(&device);
-  std::lock_guard<std::mutex> lock(kept_mutex());
-  kept().push_back(this);
-}
-MoState::~MoState() {
-  {
-    std::lock_guard<std::mutex> lock(kept_mutex());
-    kept().erase(std::find(kept().begin(), kept().end(), this));
-  }
-  cudaFree(work);
-  if (blas) cublasDestroy(blas);
-}
-// Frees idle workspaces on the current device until at most `most` bytes of
-// them are left; whether any went.
-bool give_back(size_t most) {
-  int device = 0;
-  cudaGetDevice(&device);
-  std::lock_guard<std::mutex> lock(kept_mutex());
-  const auto idle = [&](const MoState *s) { return s->device == device && !s->busy && s->work; };
+// Frees idle workspaces of the device until at most `most` bytes of them are
+// left; whether any went.  The pool's mutex is held.
+bool trim(Pool &p, int device, size_t most) {
   size_t bytes = 0;
-  for (const MoState *s : kept()) bytes += idle(s) ? s->count * sizeof(double) : 0;
+  for (const Workspace &w : p.idle) bytes += w.device == device ? w.words * sizeof(double) : 0;
   bool any = false;
-  for (MoState *s : kept()) {
-    if (bytes <= most) break;
-    if (!idle(s)) continue;
-    bytes -= s->count * sizeof(double);
-    cudaFree(s->work);
-    s->work = nullptr;
-    s->count = 0;
+  for (size_t k = 0; k < p.idle.size() && bytes > most;) {
+    if (p.idle[k].device != device) {
+      ++k;
+      continue;
+    }
+    bytes -= p.idle[k].words * sizeof(double);
+    cudaFree(p.idle[k].p);
+    p.idle.erase(p.idle.begin() + k);
     any = true;
   }
   return any;
 }
+// Gives the current device's idle workspaces back; whether there were any.
+bool give_back() {
+  int device = 0;
+  cudaGetDevice(&device);
+  std::lock_guard<std::mutex> lock(pool().mutex);
+  return trim(pool(), device, 0);
+}
+// The smallest idle workspace of the device that holds `words`, or none.
+Workspace take_idle(int device, size_t words) {
+  Pool &p = pool();
+  std::lock_guard<std::mutex> lock(p.mutex);
+  size_t best = p.idle.size();
+  for (size_t k = 0; k < p.idle.size(); ++k)
+    if (p.idle[k].device == device && p.idle[k].words >= words &&
+        (best == p.idle.size() || p.idle[k].words < p.idle[best].words))
+      best = k;
+  if (best == p.idle.size()) return {};
+  const Workspace w = p.idle[best];
+  p.idle.erase(p.idle.begin() + best);
+  return w;
+}
+void keep_idle(const Workspace &w) {
+  Pool &p = pool();
+  std::lock_guard<std::mutex> lock(p.mutex);
+  p.idle.push_back(w);
+  trim(p, w.device, kMoKeepBytes);
+}
+
+// What a context keeps: the cuBLAS handle.
+struct MoState {
+  cublasHandle_t blas = nullptr;
+  int device = 0;
+  MoState() {
+    cudaGetDevice(&device);
+    Pool &p = pool();
+    std::lock_guard<std::mutex> lock(p.mutex);
+    if ((int)p.users.size() <= device) p.users.resize(device + 1, 0);
+    ++p.users[device];
+  }
+  ~MoState() {
+    Pool &p = pool();
+    {
+      std::lock_guard<std::mutex> lock(p.mutex);
+      if (--p.users[device] == 0) trim(p, device, 0);
+    }
+    if (blas) cublasDestroy(blas);
+  }
+};
 MoState *context_state(hfg_ctx *ctx) {
   MoState *st = static_cast<MoState *>(hfg::ctx_handle(ctx));
   if (!st) {
@@ -189,35 +217,25 @@ MoState *context_state(hfg_ctx *ctx) {
 
 // The unpacked AO table M[(m n),(l s)] of the context (stored-mode build) and
 // the intermediates of the blocks that follow, of at most `ov_max` index pairs
-// on either side.  Holds the context's workspace while it lives.
+// on either side, in a workspace of the pool.
 struct MoTables {
   int n = 0;
   double *M = nullptr, *T = nullptr, *Y = nullptr;  // T: 2 N^2 ov_max, Y: N^2 ov_max
   long long cap = 0;
   cublasHandle_t blas = nullptr;
-  MoState *state = nullptr;
+  Workspace work;
   bool finished = false;  // nothing queued uses the tables any more
   MoTables() = default;
   MoTables(const MoTables &) = delete;
-  void hold(MoState *s) {
-    std::lock_guard<std::mutex> lock(kept_mutex());
-    state = s;
-    state->busy = true;
-  }
   ~MoTables() {
-    if (!state) return;
+    if (!work.p) return;
     if (!finished) cudaDeviceSynchronize();
-    {
-      std::lock_guard<std::mutex> lock(kept_mutex());
-      state->busy = false;
-      kept().erase(std::find(kept().begin(), kept().end(), state));
-      kept().push_back(state);
-    }
-    give_back(kMoKeepBytes);
+    if (work.words * sizeof(double) <= kMoKeepBytes) keep_idle(work);
+    else cudaFree(work.p);
   }
 };
 
-hfg_status prepare(hfg_ctx *ctx, long long ov_max, cudaStream_t s, Buffers &buf, MoTables &t, const char *who) {
+hfg_status prepare(hfg_ctx *ctx, long long ov_max, cudaStream_t s, MoTables &t, const char *who) {
   const int n = hfg_ctx_nbf(ctx);
   if (n <= 0) return hfg::fail_external(HFG_INVALID_ARG, std::string(who) + ": context without a single molecule");
   const long long nn = (long long)n * n;
@@ -226,29 +244,22 @@ hfg_status prepare(hfg_ctx *ctx, long long ov_max, cudaStream_t s, Buffers &buf,
   if (!state || cublasSetStream(state->blas, s) != CUBLAS_STATUS_SUCCESS)
     return hfg::fail_external(HFG_DEVICE_ERROR, std::string(who) + ": cuBLAS handle");
   t.blas = state->blas;
-  t.hold(state);
   const size_t words = (size_t)(nn * nn + 3 * nn * ov_max + count);  // M, T, Y, packed
-  double *all = state->work;
-  if (state->count < words) {
-    cudaFree(state->work);
-    state->work = nullptr;
-    state->count = 0;
+  t.work = take_idle(state->device, words);
+  if (!t.work.p) {
     size_t freeb = 0, totalb = 0;
     const double need = 8.0 * (double)words;
     cudaMemGetInfo(&freeb, &totalb);
-    if (need > 0.9 * (double)freeb && give_back(0)) cudaMemGetInfo(&freeb, &totalb);
+    if (need > 0.9 * (double)freeb && give_back()) cudaMemGetInfo(&freeb, &totalb);
     if (need > 0.9 * (double)freeb)
       return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": the unpacked AO table does not fit (" +
                                                     std::to_string(need / 1e9) + " GB needed)");
-    const bool keep = words * sizeof(double) <= kMoKeepBytes;
-    const cudaError_t e = keep ? hfg::device_alloc(&all, words * sizeof(double)) : buf.get(&all, words);
+    double *all = nullptr;
+    const cudaError_t e = hfg::device_alloc(&all, words * sizeof(double));
     if (e != cudaSuccess) return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": " + cudaGetErrorString(e));
-    if (keep) {
-      state->work = all;
-      state->count = words;
-    }
+    t.work = {all, words, state->device};
   }
-  t.M = all;
+  t.M = t.work.p;
   t.T = t.M + nn * nn;
   t.Y = t.T + 2 * nn * ov_max;
   double *packed = t.Y + nn * ov_max;
@@ -311,14 +322,13 @@ hfg_status finish(MoTables &t, cudaStream_t s, const char *who) {
   return HFG_OK;
 }
 
-hfg_status transform(hfg_ctx *ctx, const double *dC, int i0, int ni, int a0, int na, double *dX, cudaStream_t s,
-                     Buffers &buf) {
+hfg_status transform(hfg_ctx *ctx, const double *dC, int i0, int ni, int a0, int na, double *dX, cudaStream_t s) {
   const int n = hfg_ctx_nbf(ctx);
   if (n <= 0) return hfg::fail_external(HFG_INVALID_ARG, "hfg_mo_eri_ovov: context without a single molecule");
   if (!dC || !dX || ni < 1 || na < 1 || i0 < 0 || a0 < 0 || i0 + ni > n || a0 + na > n)
     return hfg::fail_external(HFG_INVALID_ARG, "hfg_mo_eri_ovov: orbital ranges");
   MoTables t;
-  hfg_status st = prepare(ctx, (long long)ni * na, s, buf, t, "hfg_mo_eri_ovov");
+  hfg_status st = prepare(ctx, (long long)ni * na, s, t, "hfg_mo_eri_ovov");
   if (st != HFG_OK) return st;
   st = block(t, {dC, i0, ni}, {dC, a0, na}, {dC, i0, ni}, {dC, a0, na}, dX, s, "hfg_mo_eri_ovov");
   if (st != HFG_OK) return st;
@@ -329,7 +339,7 @@ hfg_status transform(hfg_ctx *ctx, const double *dC, int i0, int ni, int a0, int
 
 cudaError_t hfg::device_alloc(void **p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && give_back(0)) {
+  if (e == cudaErrorMemoryAllocation && give_back()) {
     cudaGetLastError();
     e = cudaMalloc(p, bytes);
   }
@@ -340,8 +350,7 @@ extern "C" hfg_status hfg_mo_eri_ovov(hfg_ctx *ctx, const double *dC, int32_t i0
                                       double *dX, void *stream) {
   if (!ctx) return hfg::fail_external(HFG_INVALID_ARG, "hfg_mo_eri_ovov: null context");
   if (const hfg_status st = hfg::ctx_select(ctx); st != HFG_OK) return st;
-  Buffers buf;
-  return transform(ctx, dC, i0, ni, a0, na, dX, static_cast<cudaStream_t>(stream), buf);
+  return transform(ctx, dC, i0, ni, a0, na, dX, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" hfg_status hfg_mp2_rhf(hfg_ctx *ctx, const double *C, const double *eps, int32_t nocc, double *e_mp2) {
@@ -361,7 +370,7 @@ extern "C" hfg_status hfg_mp2_rhf(hfg_ctx *ctx, const double *C, const double *e
   if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);  // staged copies landed
   if (e == cudaSuccess) e = cudaMemset(dOut, 0, sizeof(double));
   if (e != cudaSuccess) return hfg::fail_external(HFG_OOM_BUDGET, std::string("hfg_mp2_rhf: ") + cudaGetErrorString(e));
-  hfg_status st = transform(ctx, dC, 0, nocc, nocc, nv, dX, nullptr, buf);
+  hfg_status st = transform(ctx, dC, 0, nocc, nocc, nv, dX, nullptr);
   if (st != HFG_OK) return st;
   const long long ov = (long long)nocc * nv;
   mp2_energy<<<grid_for(ov * ov), 256>>>(dX, dE, nocc, nv, dOut);
@@ -425,7 +434,7 @@ extern "C" hfg_status hfg_mp2_uhf(hfg_ctx *ctx, const double *Cp, const double *
   if (e != cudaSuccess) return hfg::fail_external(HFG_OOM_BUDGET, std::string(who) + ": " + cudaGetErrorString(e));
   cudaStream_t s = nullptr;
   MoTables t;
-  hfg_status st = prepare(ctx, ovmax, s, buf, t, who);
+  hfg_status st = prepare(ctx, ovmax, s, t, who);
   if (st != HFG_OK) return st;
   // first sum: all C+, i, j < n+, a, b >= n+
   std::vector<std::pair<Mp2Block, const double *>> blocks;
@@ -487,9 +496,8 @@ extern "C" hfg_status hfg_mo_eri_full(hfg_ctx *ctx, const double *dC, double *dX
   if (n <= 0) return hfg::fail_external(HFG_INVALID_ARG, "hfg_mo_eri_full: context without a single molecule");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (const hfg_status st = hfg::ctx_select(ctx); st != HFG_OK) return st;
-  Buffers buf;
   MoTables t;
-  hfg_status st = prepare(ctx, (long long)n * n, s, buf, t, who);
+  hfg_status st = prepare(ctx, (long long)n * n, s, t, who);
   if (st != HFG_OK) return st;
   if ((st = block(t, {dC, 0, n}, {dC, 0, n}, {dC, 0, n}, {dC, 0, n}, dX, s, who)) != HFG_OK) return st;
   return finish(t, s, who);

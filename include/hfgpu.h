@@ -244,9 +244,9 @@ hfg_status hfg_moments(const hfg_shells *shells, int32_t device, double *Mx, dou
  * getElectronElectron (IntegralsRepository.h:190-291) for that block.  Uses
  * the context's stored-mode table (its screening and ERI convention),
  * unpacked on the device: needs 9/8 nbf^4 + 3 nbf^2 ni na doubles free, else
- * HFG_OOM_BUDGET.  The context keeps that workspace for its next transform:
- * idle contexts at most 1 GiB of it together per device, which goes with the
- * context, or when an allocation of this library finds no memory.
+ * HFG_OOM_BUDGET.  The workspace is kept for the next transform on the device,
+ * at most 1 GiB of idle ones per device: they go with the last context there
+ * that ran a transform, or when an allocation of this library finds no memory.
  * Single-molecule contexts only. */
 hfg_status hfg_mo_eri_ovov(hfg_ctx *ctx, const double *dC, int32_t i0, int32_t ni, int32_t a0, int32_t na, double *dX,
                            void *stream);
