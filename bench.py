@@ -64,10 +64,10 @@ def workload():
     return Z, xyz
 
 
-# DRAM bytes (read + write) per launch of a class kernel on this workload,
-# from one ncu capture of the bench's own build, caches flushed before the
-# launch (profiles/eri_class_kernel_ps_ss_h2o32_traffic.md)
-TRAFFIC = {(1, 0, 0, 0): 26716928, (0, 0, 0, 0): 21508864}
+# DRAM bytes (read + write) per launch of a grouped class kernel on this
+# workload, from one ncu capture of the workload's build, caches flushed before
+# the launch (profiles/eri_group_kernel_h2o32_traffic.md)
+TRAFFIC = {(1, 0, 0, 0): 19859968, (0, 0, 0, 0): 20406016}
 
 # the large classes with a split path (primitive kernel, then HRR/digest)
 SPLIT_CLASSES = {(2, 1, 1, 1), (2, 1, 2, 0), (2, 1, 2, 1), (2, 2, 1, 0), (2, 2, 1, 1), (2, 2, 2, 0), (2, 2, 2, 1),
@@ -638,7 +638,7 @@ def main():
                    "function_quartets": stats_full["function_quartets"],
                    "l2": "flushed (256 MB write) between steps",
                    "grid_blocks_per_sm": grids or ("fixed 4" if args.no_streams else "fixed 1"),
-                   "large_class_kernels": paths or "default: warp for (22|22), split for the rest",
+                   "large_class_kernels": paths or "default: warp for (22|22) and classes of few quartets, split for the rest",
                    "prim_quartets_per_lane_target": tasks or "fixed 96",
                    "class_streams": 1 if args.no_streams else 13,
                    "cuda_graph": not args.no_graphs,
@@ -646,12 +646,13 @@ def main():
                    else "single GPU"},
         "e2e": {"value": e2e, "unit": "quartets/s", "h2d_bytes_per_step": n * n * 8, "d2h_bytes_per_step": n * n * 8},
         "gpu_launches": stats["kernel_launches"] * args.steps,
-        "roofline": {"bound": "fp64", "kernel": f"({top['la']}{top['lb']}|{top['lc']}{top['ld']}) J/K class kernel",
+        "roofline": {"bound": "fp64", "kernel": f"({top['la']}{top['lb']}|{top['lc']}{top['ld']}) "
+                               + ("grouped J/K class kernel" if top["grouped"] else "J/K class kernel"),
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "peak_source": "measured in-run: FP64 FMA microbenchmark (hfg_measure_fp64_peak)",
                      "flop_count": "reference recursion loops walked per class (hartreefock_b200/flops.py)",
                      "achieved_generated_code_count": achieved_gen,
-                     "traffic": TRAFFIC.get((top["la"], top["lb"], top["lc"], top["ld"])),
+                     "traffic": TRAFFIC.get((top["la"], top["lb"], top["lc"], top["ld"])) if top["grouped"] else None,
                      "traffic_unit": "DRAM bytes per launch (ncu capture of this workload, profiles/)",
                      "build": {"achieved": build_flops / world / (total_ms / args.steps / 1e3) / 1e12,
                                "frac": build_flops / world / (total_ms / args.steps / 1e3) / 1e12 / peak,
@@ -662,6 +663,7 @@ def main():
                      "tflops": round(c["flops"] / max(c["ms"], 1e-9) / 1e9, 3), "tasks": c["tasks"],
                      "lane_occupancy": round(c["lane_occupancy"], 3),
                      "kernel": "warp per quartet" if c["warp_kernel"] else
+                     "grouped: runs of bras, thread per quartet" if c["grouped"] else
                      "split: thread per quartet, then HRR/digest" if (c["la"], c["lb"], c["lc"], c["ld"]) in SPLIT_CLASSES
                      else "thread per quartet"} for c in prof],
         "clocks": clocks.summary(),

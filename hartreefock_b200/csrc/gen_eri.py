@@ -960,9 +960,11 @@ def emit_warp(out_dir):
 
 def is_group_class(la, lb, lc, ld):
     """Classes the grouped J/K kernel (eri_group.cuh) serves: contracted blocks
-    of at most 27 elements.  Above that the accumulators it keeps over a run of
-    bras spill: (dp|ps) 0.98 -> 1.17 ms, (dd|ss) 0.31 -> 0.50 per (H2O)32 build,
-    (ds|ds) 0.17 -> 0.22 per (H2O)16 build."""
+    of at most 27 elements.  The largest of them spill some of the accumulators
+    that the kernel keeps over a run of bras and still gain (RHF spill stores of
+    (ps|ps) 320 B, 1.77 -> 1.57 ms per (H2O)32 build; (ds|ps) 636 B, 2.17 ->
+    1.83; at most 136 B in the others); larger ones lose: (dp|ps) 0.98 -> 1.17
+    ms, (dd|ss) 0.31 -> 0.50, (ds|ds) 0.17 -> 0.22 per (H2O)16 build."""
     ne = sum((L + 1) * (L + 2) // 2 for L in range(la, la + lb + 1))
     nf = sum((L + 1) * (L + 2) // 2 for L in range(lc, lc + ld + 1))
     return ne * nf <= 27

@@ -88,9 +88,10 @@ __host__ __device__ constexpr bool boys_from_global_split(int la, int lb, int lc
 
 // T from which a primitive quartet of total angular momentum L counts as far:
 // there the asymptotic F_m = (2m-1)!!/(2T)^m sqrt(pi/T)/2 without the e^-T
-// terms is within 1e-16 relative of F_m for every m <= L (the missing part is
-// e^-T (2T)^(L-1) / ((2L-1)!! F_0): 8e-17 at L = 1, T = 40.5; 9e-17 at L = 4,
-// T = 48; 8e-17 at L = 8, T = 58).
+// terms is within 1.2e-16 relative, about half an ulp, of F_m for every m <= L
+// (what is missing is the regularised upper incomplete gamma function
+// Q(m + 1/2, T): 2e-17 at L = 1, T = 40.5; 1.0e-16 at L = 4, T = 48; at most
+// 1.13e-16, at L = 5 and 6; 9e-17 at L = 8, T = 58).
 __host__ __device__ constexpr double far_T(int L) { return 38.0 + 2.5 * L; }
 // Unroll factor of the grouped kernel's far loop over bra primitives.
 __host__ __device__ constexpr int far_unroll(int la, int lb, int lc, int ld) {
@@ -100,7 +101,7 @@ __host__ __device__ constexpr int far_unroll(int la, int lb, int lc, int ld) {
 // share one staged Boys slice and L1 keeps the rest of the SM's memory.
 __host__ __device__ constexpr int group_warps(int la, int lb, int lc, int ld) {
   const int n = ncart(la) * ncart(lb) * ncart(lc) * ncart(ld);
-    return n == 1 ? 24 : n <= 9 ? 16 : n == 18 ? 12 : 8;
+  return n == 1 ? 24 : n <= 9 ? 16 : n == 18 ? 12 : 8;
 }
 // Primitive quartets of a large class up to which its builds run the
 // warp-cooperative kernel, a quartet per warp, instead of the split path, a
@@ -232,7 +233,8 @@ constexpr int kGroupTaskSteps = 256;
 // 22.1 ms one after another and 25.2 -> 22.1 on streams, (H2O)16 (14,000 to
 // 153,000) 6.26 -> 5.83 and 4.99 -> 4.88, C9H20 / 6-31+G** (23,000 to 211,000)
 // 8.79 -> 8.55 but 6.94 -> 7.30, UHF C10H22 / 6-31G* (below 100,000) 5.03 -> 4.91
-// but 3.23 -> 3.57.
+// but 3.23 -> 3.57.  Shards take the line of concurrent streams whatever the
+// context's (each walks a part of the tasks, and every rank the same list).
 constexpr int kGroupMinTasks = 750;
 
 // Ket primitive pairs by list position: block `pos >> 5` of a pair class's list

@@ -124,6 +124,7 @@ const char *fake_log() { return log_.c_str(); }
 long long fake_prim_pair_bytes() {
   return sizeof(hfg::PrimPair) + sizeof(hfg::PrimPairF) + hfg::kKetFields * sizeof(double);
 }
+double fake_far_T(int L) { return hfg::far_T(L); }
 void fake_clear() {
   bad.clear();
   log_.clear();

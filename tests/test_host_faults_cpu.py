@@ -279,11 +279,21 @@ def admission_counts_the_tables_there_are(L):
         eng.close()
 
 
+def far_quartets_need_no_exponential(L):
+    """At the limit of the far form the asymptotic Boys function is off by the
+    regularised upper incomplete gamma function Q(m + 1/2, T): about half an ulp."""
+    from scipy.special import gammaincc
+    L.fake_far_T.restype = ctypes.c_double
+    for total in range(9):
+        T = L.fake_far_T(total)
+        assert max(gammaincc(m + 0.5, T) for m in range(total + 1)) < 1.2e-16
+
+
 CASES = [f.__name__ for f in (rebuild_survives_failed_allocations, context_gives_everything_back,
                               contexts_on_two_devices, grouped_runs,
                               precision_contexts_hold_no_grouped_lists, plain_builds_hold_no_compaction_lists,
                               autotuners_time_what_they_set, transform_workspaces_are_given_back,
-                              admission_counts_the_tables_there_are)]
+                              admission_counts_the_tables_there_are, far_quartets_need_no_exponential)]
 
 
 @pytest.mark.parametrize("case", CASES)
